@@ -416,11 +416,21 @@ __device__ __noinline__ void file_after_free(uint32_t sb, uint32_t before, uint3
   }
 }
 
+// Lanes of `mask` that name the same slab and hold blocks of the same n (1, 2,
+// 4 or 8) chunks: their chunks are n times the lanes.  A slab holds blocks of
+// one size almost always, so the n in the key seldom splits a group; summing
+// a slab's group whatever its n with a reduction instead costs 56 cycles for
+// one group and over 150 per group for several (a reduction serves one
+// sub-mask at a time), against 35 for the population count.
+__device__ __forceinline__ uint32_t slab_group(uint32_t mask, uint32_t sb, uint32_t n) {
+  return __match_any_sync(mask, (sb << 4) | n);
+}
+
 // Removes `n` chunks from slab sb's count, aggregated over the calling lanes
-// in `mask` that name the same slab; the group leader files the slab.
+// in `mask` that name the same slab and n; the group leader files the slab.
 __device__ __forceinline__ void count_down(uint32_t mask, uint32_t sb, uint32_t n) {
-  uint32_t grp = __match_any_sync(mask, sb);
-  uint32_t total = __reduce_add_sync(grp, n);
+  uint32_t grp = slab_group(mask, sb, n);
+  uint32_t total = __popc(grp) * n;
   if (lane_id() == (uint32_t)(__ffs(grp) - 1)) {
     uint32_t before = atom_add(ctr_of(sb), 0u - (total << kCntShift));
     file_after_free(sb, before, total);
@@ -988,12 +998,12 @@ __device__ __forceinline__ bool probe_from(uint32_t sb, const Class &c, uint64_t
 __device__ __forceinline__ bool commit(uint32_t rmask, uint32_t sb, uint32_t ncib,
                                        uint32_t cid, uint32_t busy, uint32_t pos,
                                        uint32_t block, bool &crossed) {
-  const uint32_t grp = __match_any_sync(rmask, sb);
-  const uint32_t total = __reduce_add_sync(grp, ncib);
+  const uint32_t grp = slab_group(rmask, sb, ncib);
+  const uint32_t total = __popc(grp) * ncib;
   const uint32_t lead = __ffs(grp) - 1;
   uint32_t before = 0;
   if (lane_id() == lead) before = atom_add_meta(ctr_of(sb), total << kCntShift);
-  before = __shfl_sync(grp, before, lead);
+  before = __shfl_sync(rmask, before, lead);
   const bool ok = ((before >> kChunkShift) & kChunkField) == cid;
   const uint32_t n0 = before >> kCntShift;
   crossed = n0 + total >= busy && n0 < busy;
@@ -1110,8 +1120,8 @@ __device__ __noinline__ void *malloc_slow(uint32_t warp, uint32_t hs, uint32_t n
       const bool give_back = !reserved && credit != kNone;
       const uint32_t gmask = __ballot_sync(want_mask, give_back);
       if (give_back) {
-        const uint32_t grp = __match_any_sync(gmask, credit);
-        const uint32_t total = __reduce_add_sync(grp, c.ncib);
+        const uint32_t grp = slab_group(gmask, credit, c.ncib);
+        const uint32_t total = __popc(grp) * c.ncib;
         if (me == (uint32_t)(__ffs(grp) - 1)) {
           ret_before = atom_add_meta(ctr_of(credit), 0u - (total << kCntShift));
           ret_total = total;
@@ -1169,7 +1179,7 @@ __device__ __forceinline__ uint32_t take_ticket(uint32_t mask, uint32_t hs) {
   const uint32_t lead = __ffs(grp) - 1;
   uint32_t base = 0;
   if (lane_id() == lead) base = atom_add(&g_st.ticket[hs * kTicketStride], __popc(grp));
-  base = __shfl_sync(grp, base, lead);
+  base = __shfl_sync(mask, base, lead);
   return base + __popc(grp & lanemask_lt());
 }
 
@@ -1228,7 +1238,7 @@ __device__ __forceinline__ void *malloc_small(uint32_t nbytes) {
     const uint32_t lead = __ffs(sgrp) - 1;
     if (lane_id() == lead)
       before = atom_add_meta(ctr_of(sb), (uint32_t)__popc(sgrp) << kCntShift);
-    before = __shfl_sync(sgrp, before, lead);
+    before = __shfl_sync(smask, before, lead);
   }
   if (sb == kNone) {
     flags |= kNeedHead;
@@ -1290,6 +1300,28 @@ __device__ __forceinline__ void *malloc_small(uint32_t nbytes) {
   return p;
 }
 
+__device__ __forceinline__ Desc ld_desc(const Desc *p) {
+  Desc d;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(d.size_id), "=r"(d.chunk_id), "=r"(d.is_head), "=r"(d.chunk_enc)
+               : "l"(p));
+  return d;
+}
+
+// Whether a count of n0 chunks lowered by n crosses a threshold of size sid
+// or empties the slab: only then is the slab filed anew.  sid is the size
+// that the descriptor showed at the start of the free; a slab whose size
+// changed meanwhile has the same chunk size, and thresholds that differ by
+// two chunks at most.  Saves file_after_free's own reads of the descriptor
+// (one more round trip) for nearly every free in a slab that is no head.
+__device__ __forceinline__ bool crosses(uint32_t sid, uint32_t n0, uint32_t n) {
+  if (sid >= kNSizes) return true;
+  const uint4 b = __ldg(reinterpret_cast<const uint4 *>(&g_cls[sid]) + 1);
+  const uint32_t n1 = n0 - n;  // b: sparse, hash_step, roomy, busy
+  return n1 == 0 || (n1 <= b.w && n0 > b.w) || (n1 <= b.z && n0 > b.z) ||
+         (n1 <= b.x && n0 > b.x);
+}
+
 // Small-block free for every active lane of the calling warp; `off` is the
 // block's offset from the start of the pool.  (halloc src/halloc.cu:211-230)
 // Block starts are at least 16 B apart (24-B chunks start on 8-B
@@ -1302,7 +1334,8 @@ __device__ __forceinline__ void free_small(uint64_t off) {
   // slab's chunk size
   uint32_t *nw = &nibs_of(sb)[in >> 7];
   const uint32_t sh = (in >> 2) & 28;
-  const uint32_t enc = ld_relaxed(&g_st.desc[sb].chunk_enc);
+  const Desc d = ld_desc(&g_st.desc[sb]);
+  const uint32_t enc = d.chunk_enc;
   const uint32_t old = atom_and_meta(nw, ~(15u << sh));
   const uint32_t n = (old >> sh) & 15u;
   HA_STAMP(kStFreeNibble, old ^ enc);
@@ -1312,12 +1345,13 @@ __device__ __forceinline__ void free_small(uint64_t off) {
   if (valid) red_and_meta(&bits_of(sb)[ichunk >> 5], ~(((1u << n) - 1u) << (ichunk & 31)));
   const uint32_t vmask = __ballot_sync(__activemask(), valid);
   if (valid) {
-    const uint32_t grp = __match_any_sync(vmask, sb);
-    const uint32_t total = __reduce_add_sync(grp, n);
+    const uint32_t grp = slab_group(vmask, sb, n);
+    const uint32_t total = __popc(grp) * n;
     if (lane_id() == (uint32_t)(__ffs(grp) - 1)) {
       const uint32_t before = atom_add_meta(ctr_of(sb), 0u - (total << kCntShift));
       HA_STAMP(kStFreeCount, before);
-      if (!(before & kHeadFlag)) file_after_free(sb, before, total);
+      if (!(before & kHeadFlag) && crosses(d.size_id, before >> kCntShift, total))
+        file_after_free(sb, before, total);
     }
   }
   HA_STAMP(kStFreeOut, vmask);
