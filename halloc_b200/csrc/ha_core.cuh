@@ -255,7 +255,7 @@ __device__ __forceinline__ uint32_t chunk_div(uint32_t v, uint32_t enc) {
 // ---------------------------------------------------------------------------
 // slab accessors
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t *ctr_of(uint32_t sb) { return &g_st.ctr[sb * kCtrStride]; }
+__device__ __forceinline__ uint32_t *ctr_of(uint32_t sb) { return &g_st.ctr[ctr_index(sb)]; }
 __device__ __forceinline__ uint32_t used_of(uint32_t sb) {
   return ld_meta(ctr_of(sb)) >> kCntShift;
 }
@@ -365,7 +365,7 @@ __device__ __noinline__ uint32_t set_take(uint32_t k) {
 // head that still has chunks in use, files it as sparse.  Caller holds the
 // slab lock.  (halloc src/slab.cuh:89-113)
 __device__ __noinline__ void try_release(uint32_t sb, uint32_t cid, bool from_head) {
-  Desc *d = &g_st.desc[sb];
+  Desc *d = &g_st.desc[desc_index(sb)];
   if (ld_relaxed(&d->is_head) || cid == kNone) return;
   uint32_t *c = ctr_of(sb);
   const uint32_t clear = ((kNone - cid) & kChunkField) << kChunkShift;
@@ -391,7 +391,7 @@ __device__ __noinline__ void try_release(uint32_t sb, uint32_t cid, bool from_he
 // its count dropped from n0 to n1 (halloc src/slab.cuh:161-224).
 __device__ __noinline__ void file_after_free(uint32_t sb, uint32_t before, uint32_t change) {
   if (before & kHeadFlag) return;
-  Desc *d = &g_st.desc[sb];
+  Desc *d = &g_st.desc[desc_index(sb)];
   uint32_t sid = ld_relaxed(&d->size_id), cid = ld_relaxed(&d->chunk_id);
   if (sid == kNone || cid == kNone) return;
   Class cl = load_class(sid);
@@ -443,7 +443,7 @@ __device__ __forceinline__ void count_down(uint32_t mask, uint32_t sb, uint32_t 
 // both are the reference's rules (halloc src/slab.cuh:227-255) and are kept
 // for identical set contents.
 __device__ __noinline__ void detach(uint32_t sb) {
-  Desc *d = &g_st.desc[sb];
+  Desc *d = &g_st.desc[desc_index(sb)];
   st_relaxed(&d->is_head, 0);
   uint32_t before = atom_add(ctr_of(sb), 0u - kHeadFlag);
   uint32_t n = before >> kCntShift;
@@ -465,7 +465,7 @@ __device__ __noinline__ void detach(uint32_t sb) {
 }
 
 __device__ __forceinline__ void make_head(uint32_t sb) {
-  st_relaxed(&g_st.desc[sb].is_head, 1);
+  st_relaxed(&g_st.desc[desc_index(sb)].is_head, 1);
   red_add(ctr_of(sb), kHeadFlag);
 }
 
@@ -475,7 +475,7 @@ __device__ __forceinline__ void make_head(uint32_t sb) {
 // thresholds goes to the busy set of its size, so no free space is stranded
 // outside every set.  Caller holds the slab lock.
 __device__ __noinline__ void retire(uint32_t sb) {
-  Desc *d = &g_st.desc[sb];
+  Desc *d = &g_st.desc[desc_index(sb)];
   st_relaxed(&d->is_head, 0);
   const uint32_t before = atom_add(ctr_of(sb), 0u - kHeadFlag);
   const uint32_t n = before >> kCntShift;
@@ -533,7 +533,7 @@ __device__ __noinline__ uint32_t find_slab(uint32_t sid) {
       set_put(kSetRoomy + sid, sb);
       return kNone;
     }
-    Desc *d = &g_st.desc[sb];
+    Desc *d = &g_st.desc[desc_index(sb)];
     bool found = false;
     if (!ld_relaxed(&d->is_head) && ld_relaxed(&d->size_id) == sid) {
       if (used_of(sb) <= c.roomy) {
@@ -551,7 +551,7 @@ __device__ __noinline__ uint32_t find_slab(uint32_t sid) {
       set_put(kSetSparse + cid, sb);
       return kNone;
     }
-    Desc *d = &g_st.desc[sb];
+    Desc *d = &g_st.desc[desc_index(sb)];
     bool found = false;
     if (!ld_relaxed(&d->is_head) && ld_relaxed(&d->chunk_id) == cid) {
       if (used_of(sb) <= c.sparse) {
@@ -572,7 +572,7 @@ __device__ __noinline__ uint32_t find_slab(uint32_t sid) {
       red_add(&g_st.n_free, 1u);
       return kNone;
     }
-    Desc *d = &g_st.desc[sb];
+    Desc *d = &g_st.desc[desc_index(sb)];
     bool found = false;
     if (!ld_relaxed(&d->is_head)) {
       found = true;
@@ -591,7 +591,7 @@ __device__ __noinline__ uint32_t find_slab(uint32_t sid) {
       set_put(kSetBusy + sid, sb);
       return kNone;
     }
-    Desc *d = &g_st.desc[sb];
+    Desc *d = &g_st.desc[desc_index(sb)];
     bool found = false;
     if (!ld_relaxed(&d->is_head) && ld_relaxed(&d->size_id) == sid) {
       found = true;
@@ -1334,7 +1334,7 @@ __device__ __forceinline__ void free_small(uint64_t off) {
   // slab's chunk size
   uint32_t *nw = &nibs_of(sb)[in >> 7];
   const uint32_t sh = (in >> 2) & 28;
-  const Desc d = ld_desc(&g_st.desc[sb]);
+  const Desc d = ld_desc(&g_st.desc[desc_index(sb)]);
   const uint32_t enc = d.chunk_enc;
   const uint32_t old = atom_and_meta(nw, ~(15u << sh));
   const uint32_t n = (old >> sh) & 15u;

@@ -466,9 +466,9 @@ int init_impl(const ha_opts_c &o) {
     st->committed = committed;
     st->n_free = committed;  // every backed slab starts in the free set
     for (uint32_t sb = 0; sb < nsbs; sb++) {
-      st->ctr[sb * ha::kCtrStride] = ha::kCtrInit;
-      st->desc[sb].size_id = ha::kNone;
-      st->desc[sb].chunk_id = ha::kNone;
+      st->ctr[ha::ctr_index(sb)] = ha::kCtrInit;
+      st->desc[ha::desc_index(sb)].size_id = ha::kNone;
+      st->desc[ha::desc_index(sb)].chunk_id = ha::kNone;
       if (sb >= committed) continue;  // not backed yet: in no set
       st->sets[ha::kSetFree][sb >> 5] |= 1u << (sb & 31);
       st->sums[ha::kSetFree][sb >> 10] |= 1u << ((sb >> 5) & 31);
@@ -616,7 +616,7 @@ __global__ void ha_trim_k(uint32_t ncand, uint32_t max_slabs) {
     const uint32_t sb = first + k, c = ld_relaxed(ctr_of(sb));
     ok = (c >> kCntShift) == 0 && !(c & kHeadFlag) &&
          ((c >> kChunkShift) & kChunkField) == kChunkField &&
-         !ld_relaxed(&g_st.desc[sb].is_head);
+         !ld_relaxed(&g_st.desc[ha::desc_index(sb)].is_head);
   }
   if (ok) {
     const uint32_t before = atomicAdd(&g_trim_slabs, n);
@@ -646,7 +646,7 @@ __global__ void ha_stats_k(int ideal) {
   uint32_t sb = blockIdx.x * blockDim.x + threadIdx.x;
   if (sb < c_cfg.nsbs) {
     uint32_t used = ld_relaxed(ctr_of(sb)) >> kCntShift;
-    uint32_t enc = ld_relaxed(&g_st.desc[sb].chunk_enc);
+    uint32_t enc = ld_relaxed(&g_st.desc[ha::desc_index(sb)].chunk_enc);
     uint64_t ubytes = enc ? (uint64_t)chunk_mul(used, enc) : 0;
     uint64_t sbb = 1ull << c_cfg.sb_sh;
     atomicAdd(&s_chunks, (unsigned long long)used);
@@ -654,7 +654,7 @@ __global__ void ha_stats_k(int ideal) {
     atomicAdd(&s_free, (unsigned long long)(sbb - ubytes));
     if (ideal && enc == 0) atomicAdd(&s_ideal, (unsigned long long)sbb);
     if ((ld_relaxed(&g_st.sets[kSetFree][sb >> 5]) >> (sb & 31)) & 1u) atomicAdd(&s_fslabs, 1u);
-    if (ld_relaxed(&g_st.desc[sb].is_head)) atomicAdd(&s_hslabs, 1u);
+    if (ld_relaxed(&g_st.desc[ha::desc_index(sb)].is_head)) atomicAdd(&s_hslabs, 1u);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -940,11 +940,11 @@ extern "C" int ha_dump_state_c(const ha_state_dump_t *d) {
     if (d->cached) d->cached[s] = st->cached[s];
   }
   for (uint32_t sb = 0; sb < n; sb++) {
-    if (d->counters) d->counters[sb] = st->ctr[sb * ha::kCtrStride];
-    if (d->size_id) d->size_id[sb] = st->desc[sb].size_id;
-    if (d->chunk_id) d->chunk_id[sb] = st->desc[sb].chunk_id;
-    if (d->is_head) d->is_head[sb] = st->desc[sb].is_head;
-    if (d->chunk_enc) d->chunk_enc[sb] = st->desc[sb].chunk_enc;
+    if (d->counters) d->counters[sb] = st->ctr[ha::ctr_index(sb)];
+    if (d->size_id) d->size_id[sb] = st->desc[ha::desc_index(sb)].size_id;
+    if (d->chunk_id) d->chunk_id[sb] = st->desc[ha::desc_index(sb)].chunk_id;
+    if (d->is_head) d->is_head[sb] = st->desc[ha::desc_index(sb)].is_head;
+    if (d->chunk_enc) d->chunk_enc[sb] = st->desc[ha::desc_index(sb)].chunk_enc;
   }
   if (d->sets)
     for (uint32_t k = 0; k < ha::kNSets; k++)
