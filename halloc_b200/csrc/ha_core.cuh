@@ -67,6 +67,12 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
+// may return a value that this SM read earlier in the same launch
+__device__ __forceinline__ uint32_t ld_cached(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -635,6 +641,7 @@ __device__ __noinline__ bool close_other_surges(uint32_t own) {
       const uint32_t w = ld_relaxed(&g_st.head[sid]);
       if (head_level(w) != 0) {
         st_release(&g_st.head[sid], head_word(head_slab(w), 0));
+        st_relaxed(&g_st.level[sid], 0);
         red_add(&g_st.n_surge_changes, 1);
       }
       unlock(hlock0);
@@ -676,9 +683,19 @@ __device__ __forceinline__ void surge_open(uint32_t sid) {
   if (head_slab(w) != kNone && level < kMaxLevel &&
       (uint64_t)kSurgeFreeOpen * nfree >= committed) {
     st_release(head, head_word(head_slab(w), level + 1));
+    st_relaxed(&g_st.level[sid], level + 1);
     red_add(&g_st.n_surge_changes, 1);
   }
   unlock(hlock);
+}
+
+// Tickets that size sid has given out, over its counters (modulo 2^32).
+__device__ __forceinline__ uint32_t tickets_of(uint32_t sid) {
+  uint32_t t = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < kMaxHeads; k++)
+    t += ld_relaxed(&g_st.ticket[(k * kNSizes + sid) * kTicketStride]);
+  return t;
 }
 
 // Counts k long-probe lanes of size sid, for 8 (the caller samples one warp
@@ -704,10 +721,8 @@ __device__ __noinline__ void probe_storm(uint32_t sid, uint32_t k, uint32_t c) {
     if (got) red_add(line + 2, got);
     return;
   }
-  const uint32_t tnow = ld_relaxed(&g_st.ticket[sid * kTicketStride]);
-  const uint32_t level = head_level(ld_relaxed(&g_st.head[sid]));
-  const bool storm = ((uint64_t)(tnow - ld_relaxed(line + 3)) << level) <
-                     (uint64_t)kProbeStormTickets * got;
+  const uint32_t tnow = tickets_of(sid);
+  const bool storm = tnow - ld_relaxed(line + 3) < kProbeStormTickets * got;
   st_relaxed(line + 3, tnow);
   HA_PSTAT(kPsJudge, 1);
   if (storm) HA_PSTAT(kPsStorm, 1);
@@ -800,7 +815,10 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs) {
       next = find_slab(sid);
     if (next == kNone) {
       st_relaxed(&g_st.no_slab[hs], epoch + 1u);
-      if (nlevel != level) st_release(head, head_word(cur, nlevel));
+      if (nlevel != level) {
+        st_release(head, head_word(cur, nlevel));
+        st_relaxed(&g_st.level[sid], nlevel);
+      }
       unlock(hlock);
       return none;
     }
@@ -813,9 +831,13 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs) {
       // grid: kSurgeTicketsUp each); close one when neither comes near.
       uint32_t *line = &g_st.storm[sid * kTicketStride];
       const uint32_t storm = atomicExch(line, 0u);
-      const uint32_t tnow = ld_relaxed(&g_st.ticket[sid * kTicketStride]);
-      const uint32_t tickets = tnow - ld_relaxed(line + 1);
+      const uint32_t tnow = tickets_of(sid);
+      const uint32_t tickets = (tnow - ld_relaxed(line + 1)) >> level;
       st_relaxed(line + 1, tnow);
+      // how long the old head lived (units of 1,024 ns)
+      const uint32_t tick = (uint32_t)(globaltimer_ns() >> 10);
+      const uint32_t life = tick - ld_relaxed(line + 4);
+      st_relaxed(line + 4, tick);
       const uint32_t per_set = storm >> level;
       const bool crowded = per_set >= kSurgeQueueMin && tickets < kSurgeTicketsUp * per_set;
       const bool calm = per_set < kSurgeQueueMin / 4 || tickets >= kSurgeTicketsDown * per_set;
@@ -827,12 +849,16 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs) {
           (uint64_t)kSurgeFreeOpen * nfree >= committed)
         nlevel = level + 1;
       else if (level > 0 &&
-               ((storm < kSurgeDown && calm) || (uint64_t)kSurgeFreeClose * nfree < committed))
+               ((storm < kSurgeDown && calm && life >= kSurgeCalmLife) ||
+                (uint64_t)kSurgeFreeClose * nfree < committed))
         nlevel = level - 1;
     }
     st_release(head, head_word(next, nlevel));
     red_add(&g_st.n_head_changes, 1);
-    if (nlevel != level) red_add(&g_st.n_surge_changes, 1);
+    if (nlevel != level) {
+      st_relaxed(&g_st.level[sid], nlevel);
+      red_add(&g_st.n_surge_changes, 1);
+    }
     unlock(hlock);
     if (cur != kNone) {
       if (lock(&g_st.sb_lock[cur])) {
@@ -1193,20 +1219,27 @@ __device__ __forceinline__ void *malloc_small(uint32_t nbytes) {
   const uint32_t smid = sm_id();
   HA_STAMP(kStMallocIn, smid);
   uint32_t hs = (smid & (c_cfg.nheads - 1)) * kNSizes + sid;
+  // Surge sets open for this size (set 0's word says how many): lanes on the
+  // SMs of set k > 0 take that set's head and ticket.  Which ticket counter
+  // is told by a copy of the level that this SM may cache (a line of its own:
+  // a relaxed load of a line drops it from L1), and set k's head word is read
+  // along with set 0's, so that a storm costs no second round trip and its
+  // tickets do not all pass through set 0's counter first (3,600 cycles for a
+  // ticket with nine sizes in a warp).  A stale copy only draws the ticket
+  // from another counter; the head comes from the words as they are now.
+  const uint32_t guess = ld_cached(&g_st.level[sid]);
+  const uint32_t kg = smid & ((1u << guess) - 1u);
+  const uint32_t hg = kg ? kg * kNSizes + sid : hs;
   const uint32_t w = ld_relaxed(&g_st.head[hs]);
-  uint32_t ticket = take_ticket(warp, hs);
+  const uint32_t wg = ld_relaxed(&g_st.head[hg]);
+  const uint32_t ticket = take_ticket(warp, hg);
   uint32_t sb = head_slab(w);
   HA_STAMP(kStMallocTicket, ticket ^ w);
   {
-    // surge sets open for this size (set 0's word says how many): lanes on
-    // the SMs of set k > 0 take that set's head and ticket instead, one
-    // round trip more, only while the size is under a storm
     const uint32_t k = smid & ((1u << head_level(w)) - 1u);
-    const uint32_t moved = __ballot_sync(warp, k != 0);
-    if (moved && k != 0) {
+    if (k != 0) {
       hs = k * kNSizes + sid;
-      sb = head_slab(ld_relaxed(&g_st.head[hs]));
-      ticket = take_ticket(moved, hs);
+      sb = head_slab(hs == hg ? wg : ld_relaxed(&g_st.head[hs]));
     }
   }
   const uint4 mm = __ldg(&g_mod[sid]);

@@ -74,6 +74,12 @@ constexpr uint32_t kRedirect = 0xfffffffeu;  // replace_head: use head set 0
 // of one head of set 0 (a grid of 1,024 warps can never reach it)
 constexpr uint32_t kSurgeUp = 2048;
 constexpr uint32_t kSurgeDown = 256;
+// and a level closes only after a head that lived at least this long (units
+// of 1,024 ns): a grid that allocates in bursts has a short queue at its last
+// head changes, and closing there made the next burst open the sets again
+// (256-B blocks from 1 M threads in bursts: 660 us with 25, 585 with 100 or
+// 400; a loop over all sizes 156, 130 and 148; a graph build 542, 538, 517)
+constexpr uint32_t kSurgeCalmLife = 100;
 // second trigger (off unless built with HA_SURGE_TICKETS_UP > 0): at least
 // kSurgeQueueMin warps queued per open set while the head served fewer than
 // kSurgeTicketsUp allocations per queued warp (P: 1,024 warps at most against
@@ -164,6 +170,8 @@ struct State {
   uint32_t head_lock[kMaxHeads * kNSizes * kTicketStride];
   alignas(128) uint32_t head[kMaxHeads * kNSizes];
   uint32_t cached[kMaxHeads * kNSizes];
+  // per size: a copy of the surge level, for loads that L1 may serve
+  alignas(128) uint32_t level[kTicketStride];
   alignas(128) uint32_t status;
   uint32_t wait_limit_us;
   uint32_t n_head_changes;
@@ -178,7 +186,8 @@ struct State {
   // per size, one 128-B line: [0] warps that queued for the head lock since
   // the last change of its set-0 head, capped near kSurgeUp; [1] set 0's
   // ticket at that change; [2] long-probe lanes in the current probe-storm
-  // window; [3] set 0's ticket when that window began
+  // window; [3] set 0's ticket when that window began; [4] time of the last
+  // change of its set-0 head (units of 1,024 ns)
   alignas(128) uint32_t storm[kNSizes * kTicketStride];
   alignas(128) uint32_t ctr[kMaxSlabs * kCtrStride];
   alignas(128) Desc desc[kMaxSlabs];

@@ -592,6 +592,7 @@ __global__ void ha_close_surges_k() {
       const uint32_t w = ld_relaxed(&g_st.head[sid]);
       if (head_level(w) != 0) {
         st_release(&g_st.head[sid], head_word(head_slab(w), 0));
+        st_relaxed(&g_st.level[sid], 0);
         red_add(&g_st.n_surge_changes, 1);
       }
       unlock(hlock0);
