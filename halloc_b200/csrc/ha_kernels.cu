@@ -761,12 +761,18 @@ __device__ __forceinline__ uint32_t graph_degree(uint32_t u, uint32_t seed, cons
   while (d < ncdf && cdf[d] <= h) d++;
   return d;
 }
-__device__ __forceinline__ uint32_t graph_neighbour(uint32_t u, uint32_t k, uint32_t seed,
-                                                    uint32_t n) {
-  return mix32(mix32(u ^ seed ^ 0xABCDEF01u) + k * 0x9E3779B9u) % n;
+__device__ __forceinline__ uint32_t graph_neighbour(uint32_t base, uint32_t k, uint32_t n) {
+  return mix32(base + k * 0x9E3779B9u) % n;
 }
 
 // acc: [0] failed allocations, [1] reallocations (doublings), [2] edges
+//
+// Bound by the hamalloc and hafree chains of a vertex (five and four of them
+// at degree 16).  Arrays are powers of two of at least 16 bytes and so 16-byte
+// aligned: they are filled and copied four neighbours at a time, a doubling
+// reading its old array in one round trip.  The last vector of an array may
+// hold neighbours past the degree, within its capacity.  1 M vertices of mean
+// degree 16: 400 us word by word, 282 now.
 __global__ void ha_graph_build_k(uint32_t n, uint32_t seed, const uint32_t *cdf, uint32_t ncdf,
                                  unsigned long long *arr, uint32_t *deg,
                                  unsigned long long *acc) {
@@ -774,23 +780,42 @@ __global__ void ha_graph_build_k(uint32_t n, uint32_t seed, const uint32_t *cdf,
   unsigned long long nfail = 0, ngrow = 0, nedge = 0;
   if (u < n) {
     const uint32_t d = graph_degree(u, seed, cdf, ncdf);
+    const uint32_t base = mix32(u ^ seed ^ 0xABCDEF01u);
     uint32_t cap = 2, cnt = 0;
     uint32_t *a = (uint32_t *)hamalloc(cap * sizeof(uint32_t));
     if (!a) nfail++;
-    for (uint32_t k = 0; k < d && a; k++) {
-      if (cnt == cap) {
-        uint32_t *b = (uint32_t *)hamalloc(2 * cap * sizeof(uint32_t));
-        if (!b) {
-          nfail++;
-          break;
-        }
-        for (uint32_t j = 0; j < cnt; j++) b[j] = a[j];
-        hafree(a);
-        a = b;
-        cap *= 2;
-        ngrow++;
+    if (a && d) {
+      *reinterpret_cast<uint2 *>(a) =
+          make_uint2(graph_neighbour(base, 0, n), graph_neighbour(base, 1, n));
+      cnt = min(d, 2u);
+    }
+    while (a && cnt < d) {  // the array is full
+      uint32_t *b = (uint32_t *)hamalloc(2 * cap * sizeof(uint32_t));
+      if (!b) {
+        nfail++;
+        break;
       }
-      a[cnt++] = graph_neighbour(u, k, seed, n);
+      uint32_t k = cap;  // a multiple of four but for the first doubling
+      if (cap == 2) {
+        const uint2 v = *reinterpret_cast<const uint2 *>(a);
+        *reinterpret_cast<uint4 *>(b) =
+            make_uint4(v.x, v.y, graph_neighbour(base, 2, n), graph_neighbour(base, 3, n));
+        k = 4;
+      } else {
+        const uint4 *from = reinterpret_cast<const uint4 *>(a);
+        uint4 *to = reinterpret_cast<uint4 *>(b);
+#pragma unroll 4
+        for (uint32_t j = 0; j < cap / 4; j++) to[j] = from[j];
+      }
+      hafree(a);
+      a = b;
+      cap *= 2;
+      ngrow++;
+      cnt = min(d, cap);
+      for (; k < cnt; k += 4)
+        *reinterpret_cast<uint4 *>(a + k) =
+            make_uint4(graph_neighbour(base, k, n), graph_neighbour(base, k + 1, n),
+                       graph_neighbour(base, k + 2, n), graph_neighbour(base, k + 3, n));
     }
     arr[u] = (unsigned long long)(uintptr_t)a;
     deg[u] = cnt;
@@ -801,16 +826,54 @@ __global__ void ha_graph_build_k(uint32_t n, uint32_t seed, const uint32_t *cdf,
 }
 
 // Copies each vertex's array into CSR columns at offsets[u] and frees it.
-__global__ void ha_graph_gather_k(uint32_t n, unsigned long long *arr, const uint32_t *deg,
-                                  const unsigned long long *offsets, uint32_t *cols) {
-  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= n) return;
-  uint32_t *a = (uint32_t *)(uintptr_t)arr[u];
-  if (!a) return;
-  const unsigned long long o = offsets[u];
-  for (uint32_t k = 0; k < deg[u]; k++) cols[o + k] = a[k];
-  hafree(a);
-  arr[u] = 0;
+// Half a warp copies one vertex's array at a time, 16 neighbours in a load
+// and a store, with the loads of eight vertices in flight; one thread per
+// vertex, word by word, left the lanes of a warp in 32 arrays and as many
+// sectors per access: 135 us for 16.8 M columns, 65 now (floor for the bytes
+// 21 us; the rest is the frees).
+__global__ void __launch_bounds__(128) ha_graph_gather_k(uint32_t n, unsigned long long *arr,
+                                                         const uint32_t *deg,
+                                                         const unsigned long long *offsets,
+                                                         uint32_t *cols) {
+  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+  unsigned long long a = 0, o = 0;
+  uint32_t d = 0;
+  if (u < n) {
+    a = arr[u];
+    if (a) {
+      d = deg[u];
+      o = offsets[u];
+    }
+  }
+  const uint32_t l16 = lane & 15u;
+#pragma unroll 1
+  for (uint32_t v = 0; v < 32; v += 8) {
+    uint32_t x[4], y[4], dv[4];
+    unsigned long long av[4], ov[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+      const uint32_t src = v + 2 * j + (lane >> 4);
+      av[j] = __shfl_sync(0xffffffffu, a, src);
+      ov[j] = __shfl_sync(0xffffffffu, o, src);
+      dv[j] = __shfl_sync(0xffffffffu, d, src);
+      const uint32_t *p = reinterpret_cast<const uint32_t *>((uintptr_t)av[j]);
+      if (l16 < dv[j]) x[j] = p[l16];
+      if (l16 + 16 < dv[j]) y[j] = p[l16 + 16];
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+      uint32_t *to = cols + ov[j];
+      if (l16 < dv[j]) to[l16] = x[j];
+      if (l16 + 16 < dv[j]) to[l16 + 16] = y[j];
+      const uint32_t *p = reinterpret_cast<const uint32_t *>((uintptr_t)av[j]);
+      for (uint32_t k = l16 + 32; k < dv[j]; k += 16) to[k] = p[k];
+    }
+  }
+  __syncwarp();
+  if (a) {
+    hafree((void *)(uintptr_t)a);
+    arr[u] = 0;
+  }
 }
 
 // serial replay on one thread
