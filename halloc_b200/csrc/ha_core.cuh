@@ -106,6 +106,18 @@ __device__ __forceinline__ void red_or(uint32_t *p, uint32_t v) {
 __device__ __forceinline__ void red_and(uint32_t *p, uint32_t v) {
   asm volatile("red.relaxed.gpu.global.and.b32 [%0], %1;" ::"l"(p), "r"(v));
 }
+__device__ __forceinline__ uint32_t atom_cas(uint32_t *p, uint32_t expect, uint32_t v) {
+  uint32_t o;
+  asm volatile("atom.acq_rel.gpu.global.cas.b32 %0, [%1], %2, %3;"
+               : "=r"(o) : "l"(p), "r"(expect), "r"(v) : "memory");
+  return o;
+}
+__device__ __forceinline__ uint32_t atom_exch(uint32_t *p, uint32_t v) {
+  uint32_t o;
+  asm volatile("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;"
+               : "=r"(o) : "l"(p), "r"(v) : "memory");
+  return o;
+}
 __device__ __forceinline__ void fence_acq_rel() {
   asm volatile("fence.acq_rel.gpu;" ::: "memory");
 }
@@ -511,8 +523,7 @@ __device__ __noinline__ void retire_set(uint32_t hs, bool force) {
     unlock(hlock);
     return;
   }
-  const uint32_t old = head_slab(ld_relaxed(&g_st.head[hs]));
-  st_release(&g_st.head[hs], kSlabField);
+  const uint32_t old = head_slab(atom_exch(&g_st.head[hs], kSlabField));
   cuda::atomic_ref<uint32_t, cuda::thread_scope_device> cached(g_st.cached[hs]);
   const uint32_t pre = cached.exchange(kNone, cuda::memory_order_acq_rel);
   unlock(hlock);
@@ -534,7 +545,12 @@ __device__ __noinline__ uint32_t find_slab(uint32_t sid) {
   const Class c = load_class(sid);
   const uint32_t cid = c.chunk_id;
   uint32_t sb;
-  while ((sb = set_take(kSetRoomy + sid)) != kNone) {
+  // With one summary word (pools of up to 1,024 slabs) the three sets' words
+  // are read in one round trip, and only sets that hold something are searched.
+  const bool one = c_cfg.sum_words == 1;
+  const uint32_t in_roomy = one ? ld_relaxed(set_sums(kSetRoomy + sid)) : 1u;
+  const uint32_t in_sparse = one ? ld_relaxed(set_sums(kSetSparse + cid)) : 1u;
+  while (in_roomy && (sb = set_take(kSetRoomy + sid)) != kNone) {
     if (!lock(&g_st.sb_lock[sb])) {
       set_put(kSetRoomy + sid, sb);
       return kNone;
@@ -552,7 +568,7 @@ __device__ __noinline__ uint32_t find_slab(uint32_t sid) {
     unlock(&g_st.sb_lock[sb]);
     if (found) return sb;
   }
-  while ((sb = set_take(kSetSparse + cid)) != kNone) {
+  while (in_sparse && (sb = set_take(kSetSparse + cid)) != kNone) {
     if (!lock(&g_st.sb_lock[sb])) {
       set_put(kSetSparse + cid, sb);
       return kNone;
@@ -611,6 +627,20 @@ __device__ __noinline__ uint32_t find_slab(uint32_t sid) {
   return kNone;
 }
 
+// Writes a surge level into size sid's set-0 head word, whose slab a warp may
+// be exchanging meanwhile (replace_head); true if the level was another.
+__device__ __forceinline__ bool set_level(uint32_t sid, uint32_t level) {
+  uint32_t w = ld_relaxed(&g_st.head[sid]);
+  for (;;) {
+    if (head_level(w) == level) return false;
+    const uint32_t seen = atom_cas(&g_st.head[sid], w, head_word(head_slab(w), level));
+    if (seen == w) break;
+    w = seen;
+  }
+  st_relaxed(&g_st.level[sid], level);
+  return true;
+}
+
 // Whether any surge set of size sid holds a head or a prefetched slab (also
 // a set closed by a level change whose retirement lost a race).
 __device__ __noinline__ bool surge_slabs_held(uint32_t sid) {
@@ -638,12 +668,7 @@ __device__ __noinline__ bool close_other_surges(uint32_t own) {
     uint32_t *hlock0 = &g_st.head_lock[sid * kTicketStride];
     bool closed = false;
     if (ld_relaxed(hlock0) == 0 && try_lock(hlock0)) {
-      const uint32_t w = ld_relaxed(&g_st.head[sid]);
-      if (head_level(w) != 0) {
-        st_release(&g_st.head[sid], head_word(head_slab(w), 0));
-        st_relaxed(&g_st.level[sid], 0);
-        red_add(&g_st.n_surge_changes, 1);
-      }
+      if (set_level(sid, 0)) red_add(&g_st.n_surge_changes, 1);
       unlock(hlock0);
       closed = true;
     }
@@ -682,9 +707,10 @@ __device__ __forceinline__ void surge_open(uint32_t sid) {
   const uint32_t committed = ld_relaxed(&g_st.committed);
   if (head_slab(w) != kNone && level < kMaxLevel &&
       (uint64_t)kSurgeFreeOpen * nfree >= committed) {
-    st_release(head, head_word(head_slab(w), level + 1));
-    st_relaxed(&g_st.level[sid], level + 1);
-    red_add(&g_st.n_surge_changes, 1);
+    if (atom_cas(head, w, head_word(head_slab(w), level + 1)) == w) {
+      st_relaxed(&g_st.level[sid], level + 1);
+      red_add(&g_st.n_surge_changes, 1);
+    }
   }
   unlock(hlock);
 }
@@ -729,23 +755,92 @@ __device__ __noinline__ void probe_storm(uint32_t sid, uint32_t k, uint32_t c) {
   if (storm) surge_open(sid);
 }
 
+// The surge level for size sid after a head of its set 0 was used up (set
+// `level` sets open so far), from how many warps queued for the size's heads
+// during the old head's life, how many tickets set 0 gave out meanwhile (about
+// the allocations its head served) and how long it lived.  A level opens when
+// the queue is a storm (kSurgeUp), or when it is long and the head served
+// only a few allocations per queued warp of its set (a head too small for the
+// grid: kSurgeTicketsUp each), or when a warp of several lanes (`group`) used up a
+// head that lived only briefly; one closes when nothing comes near and the
+// head lived long.
+__device__ __forceinline__ uint32_t judge_level(uint32_t sid, uint32_t level, bool group) {
+  uint32_t *line = &g_st.storm[sid * kTicketStride];
+  const uint32_t storm = atomicExch(line, 0u);
+  const uint32_t tnow = ld_relaxed(&g_st.ticket[sid * kTicketStride]);
+  const uint32_t tickets = tnow - ld_relaxed(line + 1);
+  st_relaxed(line + 1, tnow);
+  // how long the old head lived (units of 1,024 ns)
+  const uint32_t tick = (uint32_t)(globaltimer_ns() >> 10);
+  const uint32_t life = tick - ld_relaxed(line + 4);
+  st_relaxed(line + 4, tick);
+  const uint32_t per_set = storm >> level;
+  const bool crowded = per_set >= kSurgeQueueMin && tickets < kSurgeTicketsUp * per_set;
+  const bool calm = per_set < kSurgeQueueMin / 4 || tickets >= kSurgeTicketsDown * per_set;
+  // more heads hold more partly filled slabs: open a level only while a
+  // quarter of the pool is free, and close one when under an eighth is
+  const uint32_t nfree = ld_relaxed(&g_st.n_free);
+  const uint32_t committed = ld_relaxed(&g_st.committed);
+  const bool hot = group && life < kSurgeHotLife;
+  if ((storm >= kSurgeUp || crowded || hot) && level < kMaxLevel &&
+      (uint64_t)kSurgeFreeOpen * nfree >= committed)
+    return level + 1;
+  if (level > 0 && ((storm < kSurgeDown && calm && life >= kSurgeCalmLife) ||
+                    (uint64_t)kSurgeFreeClose * nfree < committed))
+    return level - 1;
+  return level;
+}
+
+// What follows a change of head slot hs from slab `old` to `next`: the old
+// head is filed, the surge level judged (set 0), and the next slab
+// prefetched, the reference's steps in the reference's order.
+__device__ __noinline__ void after_change(uint32_t hs, uint32_t old, uint32_t wnew, bool judge,
+                                          bool group) {
+  const uint32_t sid = hs % kNSizes;
+  red_add(&g_st.n_head_changes, 1);
+  if (old != kNone && lock(&g_st.sb_lock[old])) {
+    detach(old);
+    unlock(&g_st.sb_lock[old]);
+  }
+  const uint32_t pre = find_slab(sid);
+  if (pre != kNone) hand_back(hs, pre);
+  if (judge) {
+    const uint32_t level = head_level(wnew), nlevel = judge_level(sid, level, group);
+    // given up when the head changed meanwhile: that change is judged itself
+    if (nlevel != level &&
+        atom_cas(&g_st.head[hs], wnew, head_word(head_slab(wnew), nlevel)) == wnew) {
+      st_relaxed(&g_st.level[sid], nlevel);
+      red_add(&g_st.n_surge_changes, 1);
+      // a level closed: retire the heads of its sets
+      for (uint32_t k = 1u << nlevel; k < (1u << level); k++)
+        retire_set(k * kNSizes + sid, false);
+    }
+  }
+}
+
 // Gives head slot hs (= set * kNSizes + size id) a new head slab once the
 // current one has reached the busy threshold: the prefetched ("cached") slab
 // first, then a search; the next slab is prefetched right away.  One lane
-// per warp calls this.  A caller that loses the race for the slot's lock
-// waits (bounded) until the head changes or the lock is released (halloc
+// per warp calls this.  `crossed` is the slab whose count the caller saw
+// cross the threshold, kNone for a caller that found no block (halloc
 // src/slab.cuh:378-445).
 //
-// The lock covers only the switch of the head.  Filing the old head and
-// prefetching the next slab, which the reference also does under the lock,
-// run after it is released, so other warps can use the new head meanwhile;
-// a single thread still performs the reference's steps in the reference's
-// order.  Two prefetches can then overlap: the loser hands its slab back.
+// The change itself is an exchange of the prefetched slab out of its slot and
+// a compare-and-swap of the head word, without the slot's lock: two dependent
+// round trips for the warp whose count crossed the threshold (the loads and
+// the exchange go out together).  Under the lock, with the level judged before
+// the new head was published, it took six, while thousands of warps waited
+// (a call here took 32,000 cycles in the serving loop and 41,000 in the phase
+// workload, 9,000 now).  The lock covers only searches, when no slab was prefetched: a caller
+// that loses the race for it waits (bounded) until the head changes or the
+// lock is released.  Filing the old head and prefetching follow the change; a
+// single thread still performs the reference's steps in the reference's order.
+// Two prefetches can overlap: the loser hands its slab back.
 //
 // Surge sets (c_cfg.surge): when thousands of warps queue for one size's
-// head (a grid far larger than its head's free space), the lock holder of
-// set 0 opens more head sets for the size, each serving the SMs whose id
-// modulo 2^level names it, and closes them again as the queue shrinks.  The
+// head (a grid far larger than its head's free space), set 0's changes open
+// more head sets for the size, each serving the SMs whose id modulo 2^level
+// names it, and close them again as the queue shrinks (judge_level).  The
 // level travels in set 0's head word.  A set-k slot answers kRedirect (use
 // set 0) when the set is closed or finds no slab; when set 0 itself finds no
 // slab while surge sets are open, it closes them all (their heads are filed
@@ -753,39 +848,71 @@ __device__ __noinline__ void probe_storm(uint32_t sid, uint32_t k, uint32_t c) {
 // one head.  A lone thread never waits for a lock, so it never opens a set
 // and gets exactly the reference's addresses.  (Probing storms open levels
 // between head changes: probe_storm above.)
-__device__ __noinline__ uint32_t replace_head(uint32_t hs) {
+__device__ __noinline__ uint32_t replace_head(uint32_t hs, uint32_t crossed, bool group) {
   const uint32_t sid = hs % kNSizes, set = hs / kNSizes;
   const bool surge_set = c_cfg.surge && set != 0;
+  const bool judge = c_cfg.surge && set == 0;
   const uint32_t none = surge_set ? kRedirect : kNone;  // "no head" answer
   uint32_t *head = &g_st.head[hs];
   uint32_t *hlock = &g_st.head_lock[hs * kTicketStride];
-  cuda::atomic_ref<uint32_t, cuda::thread_scope_device> cached(g_st.cached[hs]);
+  uint32_t *cached = &g_st.cached[hs];
   const uint32_t busy = load_class(sid).busy;
-  // One round trip for the head, the memo below, the lock word and (surge
-  // sets) set 0's head word (test before test-and-set: while the lock is
-  // held, waiting warps only read).
+  // One round trip for the head, the memo below, the lock word, the prefetched
+  // slab and (surge sets) set 0's head word.
   const uint32_t wseen = ld_relaxed(head);
   const uint32_t epoch = ld_relaxed(&g_st.set_epoch);
   const uint32_t memo = ld_relaxed(&g_st.no_slab[hs]);
   const uint32_t held = ld_relaxed(hlock);
   const uint32_t w0 = surge_set ? ld_relaxed(&g_st.head[sid]) : 0u;
+  const uint32_t ready = ld_relaxed(cached);
+  uint32_t next = crossed != kNone ? atom_exch(cached, kNone) : kNone;
   const uint32_t seen = head_slab(wseen);
-  if (surge_set && set >= (1u << head_level(w0))) return kRedirect;
-  // A failed search leaves every set it looked at empty, so until a slab is
-  // filed somewhere (set_epoch moves) another search would fail the same
-  // way: answer at once instead of queueing for the lock to search again.
-  if (memo == epoch + 1u && (seen == kNone || used_of(seen) >= busy)) return none;
+  if (surge_set && set >= (1u << head_level(w0))) {
+    if (next != kNone && lock(&g_st.sb_lock[next])) {
+      retire(next);
+      unlock(&g_st.sb_lock[next]);
+    }
+    return kRedirect;
+  }
+  if (crossed != kNone && seen != crossed) {  // changed already
+    if (next != kNone) hand_back(hs, next);
+    return seen == kNone ? none : seen;
+  }
+  if (crossed == kNone) {
+    // A failed search leaves every set it looked at empty, so until a slab is
+    // filed somewhere (set_epoch moves) another search would fail the same
+    // way: answer at once instead of queueing for the lock to search again.
+    if (memo == epoch + 1u && (seen == kNone || used_of(seen) >= busy)) return none;
+    if (seen != kNone) {
+      const uint32_t n_seen = used_of(seen);
+      if (ready != kNone) next = atom_exch(cached, kNone);
+      if (n_seen < busy) {
+        // not busy after all (the reference's re-check): hand the slab back
+        if (next != kNone) hand_back(hs, next);
+        return seen;
+      }
+    }
+  }
+  if (next != kNone) {
+    const uint32_t wnew = head_word(next, head_level(wseen));
+    const uint32_t was = atom_cas(head, wseen, wnew);
+    if (was == wseen) {
+      after_change(hs, seen, wnew, judge, group);
+      return next;
+    }
+    hand_back(hs, next);
+    const uint32_t now = head_slab(was);
+    if (now != kNone && now != seen) return now;
+    // closed meanwhile, or only the level changed: the caller comes again
+    return now == kNone ? none : now;
+  }
   if (held == 0 && try_lock(hlock)) {
-    // Under the lock, one round trip again: the head as it is now, the count
-    // of the head seen before (nearly always still the head), set 0's word
-    // (surge sets) and the prefetched slab, taken on the expectation that
-    // the head is replaced.  The exchange comes last so that its acquire
-    // does not hold up the loads.
+    // Under the lock, one round trip again: the head and set 0's word (surge
+    // sets) as they are now and a slab prefetched meanwhile.
     const uint32_t wcur = ld_relaxed(head);
-    const uint32_t cur = head_slab(wcur);
-    const uint32_t n_seen = seen != kNone ? used_of(seen) : 0u;
     const uint32_t w0now = surge_set ? ld_relaxed(&g_st.head[sid]) : 0u;
-    uint32_t next = cached.exchange(kNone, cuda::memory_order_acquire);
+    next = atom_exch(cached, kNone);
+    const uint32_t cur = head_slab(wcur);
     if (surge_set && set >= (1u << head_level(w0now))) {
       // the set closed while this warp came for its lock
       unlock(hlock);
@@ -795,91 +922,54 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs) {
       }
       return kRedirect;
     }
-    if (cur != kNone && (cur == seen ? n_seen : used_of(cur)) < busy) {
-      // not busy after all (the reference's re-check): hand the slab back
+    if (cur != seen && cur != kNone && used_of(cur) < busy) {
       if (next != kNone) hand_back(hs, next);
       unlock(hlock);
       return cur;
     }
-    const uint32_t level = set == 0 ? head_level(wcur) : 0u;
+    const uint32_t level = judge ? head_level(wcur) : 0u;
     uint32_t nlevel = level;
     if (next == kNone) next = find_slab(sid);
-    if (next == kNone && set == 0 && c_cfg.surge && surge_slabs_held(sid)) {
+    if (next == kNone && judge && surge_slabs_held(sid)) {
       // short of slabs while surge sets hold heads: close them all, which
       // files their heads and prefetched slabs where this search finds them
       for (uint32_t k = 1; k < kMaxHeads; k++) retire_set(k * kNSizes + sid, true);
       nlevel = 0;
       next = find_slab(sid);
     }
-    if (next == kNone && set == 0 && c_cfg.surge && close_other_surges(sid))
-      next = find_slab(sid);
+    if (next == kNone && judge && close_other_surges(sid)) next = find_slab(sid);
     if (next == kNone) {
       st_relaxed(&g_st.no_slab[hs], epoch + 1u);
-      if (nlevel != level) {
-        st_release(head, head_word(cur, nlevel));
-        st_relaxed(&g_st.level[sid], nlevel);
-      }
+      if (nlevel != level) set_level(sid, nlevel);
       unlock(hlock);
       return none;
     }
-    if (set == 0 && c_cfg.surge && nlevel == level) {
-      // How many warps queued for this size's heads during the old head's
-      // life, and how many tickets set 0 gave out meanwhile (about the
-      // allocations its head served).  Open a level when the queue is a
-      // storm (kSurgeUp), or when it is long and the head served only a few
-      // allocations per queued warp of its set (a head too small for the
-      // grid: kSurgeTicketsUp each); close one when neither comes near.
-      uint32_t *line = &g_st.storm[sid * kTicketStride];
-      const uint32_t storm = atomicExch(line, 0u);
-      const uint32_t tnow = tickets_of(sid);
-      const uint32_t tickets = (tnow - ld_relaxed(line + 1)) >> level;
-      st_relaxed(line + 1, tnow);
-      // how long the old head lived (units of 1,024 ns)
-      const uint32_t tick = (uint32_t)(globaltimer_ns() >> 10);
-      const uint32_t life = tick - ld_relaxed(line + 4);
-      st_relaxed(line + 4, tick);
-      const uint32_t per_set = storm >> level;
-      const bool crowded = per_set >= kSurgeQueueMin && tickets < kSurgeTicketsUp * per_set;
-      const bool calm = per_set < kSurgeQueueMin / 4 || tickets >= kSurgeTicketsDown * per_set;
-      // more heads hold more partly filled slabs: open a level only while a
-      // quarter of the pool is free, and close one when under an eighth is
-      const uint32_t nfree = ld_relaxed(&g_st.n_free);
-      const uint32_t committed = ld_relaxed(&g_st.committed);
-      if ((storm >= kSurgeUp || crowded) && level < kMaxLevel &&
-          (uint64_t)kSurgeFreeOpen * nfree >= committed)
-        nlevel = level + 1;
-      else if (level > 0 &&
-               ((storm < kSurgeDown && calm && life >= kSurgeCalmLife) ||
-                (uint64_t)kSurgeFreeClose * nfree < committed))
-        nlevel = level - 1;
-    }
-    st_release(head, head_word(next, nlevel));
-    red_add(&g_st.n_head_changes, 1);
+    const uint32_t wnew = head_word(next, nlevel);
+    const uint32_t was = head_slab(atom_exch(head, wnew));
     if (nlevel != level) {
       st_relaxed(&g_st.level[sid], nlevel);
       red_add(&g_st.n_surge_changes, 1);
     }
     unlock(hlock);
-    if (cur != kNone) {
-      if (lock(&g_st.sb_lock[cur])) {
-        detach(cur);
-        unlock(&g_st.sb_lock[cur]);
+    if (was != cur && was != kNone) {
+      // another warp's change came in between: its head may not be busy yet
+      if (lock(&g_st.sb_lock[was])) {
+        retire(was);
+        unlock(&g_st.sb_lock[was]);
       }
+      after_change(hs, kNone, wnew, judge && nlevel == level, group);
+    } else {
+      after_change(hs, was, wnew, judge && nlevel == level, group);
     }
-    // a level closed by the storm count: retire the heads of its sets
-    for (uint32_t k = 1u << nlevel; k < (1u << level) && nlevel < level; k++)
-      retire_set(k * kNSizes + sid, false);
-    const uint32_t pre = find_slab(sid);
-    if (pre != kNone) hand_back(hs, pre);
     return next;
   }
-  // Every warp that found the head busy waits here, thousands at once when a
-  // grid storms one size.  Their polls all go to the sectors of the head and
-  // lock words, which the lock holder must write to end the wait, so they
-  // back off to about a microsecond and read the lock word only every
-  // fourth poll (the head word is what normally changes).  With surge sets
-  // on, each waiting warp is counted once (up to the threshold) for the
-  // lock holder's next decision.
+  // Every warp that found the head busy and no slab prefetched waits here,
+  // thousands at once when a grid storms one size.  Their polls all go to the
+  // sectors of the head and lock words, which the lock holder must write to
+  // end the wait, so they back off to about a microsecond and read the lock
+  // word only every fourth poll (the head word is what normally changes).
+  // With surge sets on, each waiting warp is counted once (up to the
+  // threshold) for the next decision.
   if (c_cfg.surge) {
     uint32_t *storm = &g_st.storm[sid * kTicketStride];
     if (ld_relaxed(storm) < kSurgeUp) red_add(storm, 1u);
@@ -1101,7 +1191,7 @@ __device__ __noinline__ void *malloc_slow(uint32_t warp, uint32_t hs, uint32_t n
       uint32_t nsb = 0;
       if (me == lead) {
         HA_PSTAT(kPsHead, 1);
-        nsb = replace_head(hs);
+        nsb = replace_head(hs, p ? sb : kNone, (warp & (warp - 1)) != 0);
       }
       nsb = __shfl_sync(warp, nsb, lead);
       if (need_head && hs == lhs) {

@@ -74,12 +74,18 @@ constexpr uint32_t kRedirect = 0xfffffffeu;  // replace_head: use head set 0
 // of one head of set 0 (a grid of 1,024 warps can never reach it)
 constexpr uint32_t kSurgeUp = 2048;
 constexpr uint32_t kSurgeDown = 256;
-// and a level closes only after a head that lived at least this long (units
-// of 1,024 ns): a grid that allocates in bursts has a short queue at its last
-// head changes, and closing there made the next burst open the sets again
-// (256-B blocks from 1 M threads in bursts: 660 us with 25, 585 with 100 or
-// 400; a loop over all sizes 156, 130 and 148; a graph build 542, 538, 517)
-constexpr uint32_t kSurgeCalmLife = 100;
+// A head that warps of several lanes used up within kSurgeHotLife (units of
+// 1,024 ns) opens a level, too: head changes are quick enough that hardly a
+// warp queues, while the words of one head and its tickets stay hot.  A level
+// closes only after a head that lived kSurgeCalmLife and left a short queue:
+// every level doubles the life of a head, and bursts end with short queues, so
+// a limit near the first made levels open and close all the time.  Measured
+// with 32 / 100, 32 / 1,000 and 64 / 1,000: graph build 371, 345 and 345 us,
+// loop over all sizes 149, 115 and 115, private 8..3072 B 405, 374 and 375,
+// phases 2,225, 2,260 and 2,140, serving 75, 71 and 72 ms; without the first
+// rule and 100: 373, 153, 448, 2,210 us and 95 ms.
+constexpr uint32_t kSurgeHotLife = 64;
+constexpr uint32_t kSurgeCalmLife = 1000;
 // second trigger (off unless built with HA_SURGE_TICKETS_UP > 0): at least
 // kSurgeQueueMin warps queued per open set while the head served fewer than
 // kSurgeTicketsUp allocations per queued warp (P: 1,024 warps at most against
