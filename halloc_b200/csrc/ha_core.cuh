@@ -52,6 +52,9 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
   return m;
 }
+// Whether this lane is the first of group `grp` it belongs to (three times
+// quicker than comparing its id with the group's lowest set bit).
+__device__ __forceinline__ bool first_of(uint32_t grp) { return (grp & lanemask_lt()) == 0; }
 __device__ __forceinline__ uint32_t sm_id() {
   uint32_t v;
   asm("mov.u32 %0, %%smid;" : "=r"(v));
@@ -449,7 +452,7 @@ __device__ __forceinline__ uint32_t slab_group(uint32_t mask, uint32_t sb, uint3
 __device__ __forceinline__ void count_down(uint32_t mask, uint32_t sb, uint32_t n) {
   uint32_t grp = slab_group(mask, sb, n);
   uint32_t total = __popc(grp) * n;
-  if (lane_id() == (uint32_t)(__ffs(grp) - 1)) {
+  if (first_of(grp)) {
     uint32_t before = atom_add(ctr_of(sb), 0u - (total << kCntShift));
     file_after_free(sb, before, total);
   }
@@ -1118,7 +1121,7 @@ __device__ __forceinline__ bool commit(uint32_t rmask, uint32_t sb, uint32_t nci
   const uint32_t total = __popc(grp) * ncib;
   const uint32_t lead = __ffs(grp) - 1;
   uint32_t before = 0;
-  if (lane_id() == lead) before = atom_add_meta(ctr_of(sb), total << kCntShift);
+  if (first_of(grp)) before = atom_add_meta(ctr_of(sb), total << kCntShift);
   before = __shfl_sync(rmask, before, lead);
   const bool ok = ((before >> kChunkShift) & kChunkField) == cid;
   const uint32_t n0 = before >> kCntShift;
@@ -1238,7 +1241,7 @@ __device__ __noinline__ void *malloc_slow(uint32_t warp, uint32_t hs, uint32_t n
       if (give_back) {
         const uint32_t grp = slab_group(gmask, credit, c.ncib);
         const uint32_t total = __popc(grp) * c.ncib;
-        if (me == (uint32_t)(__ffs(grp) - 1)) {
+        if (first_of(grp)) {
           ret_before = atom_add_meta(ctr_of(credit), 0u - (total << kCntShift));
           ret_total = total;
           ret_sb = credit;
@@ -1275,7 +1278,7 @@ __device__ __noinline__ void *malloc_slow(uint32_t warp, uint32_t hs, uint32_t n
       const uint32_t lmask = __ballot_sync(warp, long_probe);
       if (long_probe) {
         const uint32_t grp = __match_any_sync(lmask, sid);
-        if (me == (uint32_t)(__ffs(grp) - 1)) probe_storm(sid, __popc(grp), c);
+        if (first_of(grp)) probe_storm(sid, __popc(grp), c);
       }
     }
   }
@@ -1288,22 +1291,9 @@ __device__ __noinline__ void *malloc_slow(uint32_t warp, uint32_t hs, uint32_t n
 // else (further probes, head replacement, exhaustion) continues in
 // malloc_slow exactly where the reference's loop would.
 // (halloc src/halloc.cu:125-182)
-// Tickets of head slot hs for the lanes of `mask` that name it: consecutive
-// values in lane order, one atomic per slot and warp.
-__device__ __forceinline__ uint32_t take_ticket(uint32_t mask, uint32_t hs) {
-  const uint32_t grp = __match_any_sync(mask, hs);
-  const uint32_t lead = __ffs(grp) - 1;
-  uint32_t base = 0;
-  if (lane_id() == lead) base = atom_add(&g_st.ticket[hs * kTicketStride], __popc(grp));
-  base = __shfl_sync(mask, base, lead);
-  return base + __popc(grp & lanemask_lt());
-}
-
 __device__ __forceinline__ void *malloc_small(uint32_t nbytes) {
   const uint32_t warp = __activemask();
   const uint32_t sid = size_class(nbytes);
-  const uint4 ca = __ldg(reinterpret_cast<const uint4 *>(&g_cls[sid]));
-  const uint32_t nchunks = ca.x, enc = ca.y, cid = ca.z, ncib = ca.w;
   // head slot: fixed head set of this SM with ha_set_heads_c (set 0 with the
   // reference's single head); head word and ticket in one round trip
   const uint32_t smid = sm_id();
@@ -1318,51 +1308,55 @@ __device__ __forceinline__ void *malloc_small(uint32_t nbytes) {
   // ticket with nine sizes in a warp).  A stale copy only draws the ticket
   // from another counter; the head comes from the words as they are now.
   const uint32_t guess = ld_cached(&g_st.level[sid]);
+  uint32_t w = ld_relaxed(&g_st.head[hs]);
+  // the lanes of each size draw consecutive tickets, in lane order, with one
+  // atomic, and use the head that their first lane read: one group serves
+  // the ticket and the count
+  const uint32_t grp = __match_any_sync(warp, sid);
+  const uint32_t lead = __ffs(grp) - 1, g = __popc(grp);
   const uint32_t kg = smid & ((1u << guess) - 1u);
   const uint32_t hg = kg ? kg * kNSizes + sid : hs;
-  const uint32_t w = ld_relaxed(&g_st.head[hs]);
   const uint32_t wg = ld_relaxed(&g_st.head[hg]);
-  const uint32_t ticket = take_ticket(warp, hg);
+  uint32_t ticket = 0;
+  if (first_of(grp)) ticket = atom_add(&g_st.ticket[hg * kTicketStride], g);
+  const uint4 ca = __ldg(reinterpret_cast<const uint4 *>(&g_cls[sid]));
+  const uint32_t nchunks = ca.x, enc = ca.y, cid = ca.z, ncib = ca.w;
+  w = __shfl_sync(warp, w, lead);
   uint32_t sb = head_slab(w);
-  HA_STAMP(kStMallocTicket, ticket ^ w);
-  {
-    const uint32_t k = smid & ((1u << head_level(w)) - 1u);
+  const uint32_t k = smid & ((1u << head_level(w)) - 1u);
+  if (__any_sync(warp, k != 0)) {
     if (k != 0) {
       hs = k * kNSizes + sid;
       sb = head_slab(hs == hg ? wg : ld_relaxed(&g_st.head[hs]));
     }
+    sb = __shfl_sync(warp, sb, lead);
   }
-  const uint4 mm = __ldg(&g_mod[sid]);
-  const uint64_t mn = mod_magic(mm.x, mm.y);
-  const uint32_t first = first_probe(sid, ticket, ncib, mn, nchunks);
-  const uint32_t block = (1u << ncib) - 1u;
-  HA_PSTAT(kPsAlloc, 1);
-
-  uint32_t pos = first, round = 0, flags = kWant;
-  bool reserved = false;
-  // The reservation's atomic, and for a one-chunk size (c_cfg.spec_mask) the
-  // slab count's as well, one per (warp, slab), in the same round trip: the
-  // count is added before the reservation is known to have succeeded.  Only
+  // The slab count goes out with the reservation's atomic, before it is known
+  // to have succeeded, for a one-chunk size (c_cfg.spec_mask).  Only
   // while the size has no surge set open: under a storm the counts of
   // reservations that failed would swell a head's count for a look-ahead
   // round, and the probing-storm trigger reads that count.
   const bool spec = sb != kNone && head_level(w) == 0 && ((c_cfg.spec_mask >> sid) & 1u);
+  const uint32_t smask = __ballot_sync(warp, spec);
+  const uint4 mm = __ldg(&g_mod[sid]);
+  const uint64_t mn = mod_magic(mm.x, mm.y);
+  const uint32_t block = (1u << ncib) - 1u;
+  ticket = __shfl_sync(warp, ticket, lead) + __popc(grp & lanemask_lt());
+  HA_STAMP(kStMallocTicket, ticket ^ w);
+  const uint32_t first = first_probe(sid, ticket, ncib, mn, nchunks);
+  HA_PSTAT(kPsAlloc, 1);
+
+  uint32_t pos = first, round = 0, flags = kWant;
+  bool reserved = false;
   uint32_t *bw = nullptr;
-  uint32_t mask = 0, old = 0;
+  uint32_t mask = 0, old = 0, before = 0;
   if (sb != kNone) {
     mask = block << (pos & 31);
     bw = &bits_of(sb)[pos >> 5];
     old = atom_or_meta(bw, mask);
   }
-  const uint32_t smask = __ballot_sync(warp, spec);
-  uint32_t sgrp = 0, before = 0;
-  if (spec) {
-    sgrp = __match_any_sync(smask, sb);
-    const uint32_t lead = __ffs(sgrp) - 1;
-    if (lane_id() == lead)
-      before = atom_add_meta(ctr_of(sb), (uint32_t)__popc(sgrp) << kCntShift);
-    before = __shfl_sync(smask, before, lead);
-  }
+  if (spec && first_of(grp)) before = atom_add_meta(ctr_of(sb), g << kCntShift);
+  const uint32_t busy = __ldg(&g_cls[sid].busy);
   if (sb == kNone) {
     flags |= kNeedHead;
   } else {
@@ -1379,38 +1373,35 @@ __device__ __forceinline__ void *malloc_small(uint32_t nbytes) {
       flags |= kMidRound;
     }
   }
+  // the count of the other sizes: the blocks that their groups reserved
+  uint32_t total = g, src = lead;
+  if (smask != warp) {
+    const uint32_t rgrp = __ballot_sync(warp, reserved && !spec) & grp;
+    if (!spec) {
+      total = __popc(rgrp) * ncib;
+      src = rgrp ? __ffs(rgrp) - 1 : 0;
+      if (reserved && first_of(rgrp)) before = atom_add_meta(ctr_of(sb), total << kCntShift);
+    }
+  }
+  before = __shfl_sync(warp, before, src);
   void *p = nullptr;
-  if (spec) {
-    // the early count: as commit() below, for the whole group at once.  A
-    // lane whose reservation failed hands its chunk of count to the slow
-    // path as a credit (kCredit), with whether the early count crossed the
+  if (spec || reserved) {
+    // A lane whose reservation failed hands its chunk of the early count to
+    // the slow path as a credit (kCredit), with whether that count crossed the
     // busy threshold; so does a lane whose slab changed chunk size under it
     // (its block goes back here), which asks for a new head at once (no
     // call here, so hamalloc's frame stays small).
     HA_STAMP(kStMallocCount, before);
-    const uint32_t n0 = before >> kCntShift, total = __popc(sgrp);
-    const uint32_t busy = __ldg(&g_cls[sid].busy);
+    const uint32_t n0 = before >> kCntShift;
     const bool crossed = n0 + total >= busy && n0 < busy;
     if (((before >> kChunkShift) & kChunkField) != cid) {
       if (reserved) red_and_meta(bw, ~mask);
-      reserved = false;
       flags = kWant | kNeedHead | kCredit;
     } else if (reserved) {
-      p = publish(sb, pos, enc, 1u);
-      flags = crossed ? kNeedHead : 0;
-    } else {
-      flags |= kCredit | (crossed ? kCreditCrossed : 0u);
-    }
-  }
-  const uint32_t rmask = __ballot_sync(warp, reserved && !spec);
-  if (reserved && !spec) {
-    bool crossed;
-    if (commit(rmask, sb, ncib, cid, __ldg(&g_cls[sid].busy), pos, block, crossed)) {
-      HA_STAMP(kStMallocCount, crossed);
       p = publish(sb, pos, enc, ncib);
       flags = crossed ? kNeedHead : 0;
     } else {
-      flags = kWant | kNeedHead | kCredit;
+      flags |= kCredit | (crossed ? kCreditCrossed : 0u);
     }
   }
   if (__any_sync(warp, flags != 0)) {
@@ -1470,7 +1461,7 @@ __device__ __forceinline__ void free_small(uint64_t off) {
   if (valid) {
     const uint32_t grp = slab_group(vmask, sb, n);
     const uint32_t total = __popc(grp) * n;
-    if (lane_id() == (uint32_t)(__ffs(grp) - 1)) {
+    if (first_of(grp)) {
       const uint32_t before = atom_add_meta(ctr_of(sb), 0u - (total << kCntShift));
       HA_STAMP(kStFreeCount, before);
       if (!(before & kHeadFlag) && crosses(d.size_id, before >> kCntShift, total))
