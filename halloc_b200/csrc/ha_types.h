@@ -60,15 +60,17 @@ HA_HD uint32_t desc_index(uint32_t sb) {
   return ((sb & (kMaxSlabs / 8 - 1)) << 3) | (sb / (kMaxSlabs / 8));
 }
 constexpr uint32_t kMaxRounds = 1u << 16;  // outer-loop bound of one hamalloc
-constexpr uint32_t kMaxHeads = 8;          // head slabs per size (1 = the reference policy)
+constexpr uint32_t kMaxHeads = 16;         // head slabs per size with every surge set open
+constexpr uint32_t kMaxFixedHeads = 8;     // ha_set_heads_c (1 = the reference policy)
 constexpr uint32_t kDefaultWaitUs = 1000000;  // 1 s
 
 // head words: slab id in bits 0-27 (all ones = no head), and in the word of
-// head set 0 the surge level in bits 28-29: 2^level head sets are open for
+// head set 0 the surge level in bits 28-30: 2^level head sets are open for
 // the size (level 0 = the reference's single head)
 constexpr uint32_t kSlabField = 0x0fffffffu;
 constexpr uint32_t kLevelShift = 28;
-constexpr uint32_t kMaxLevel = 3;          // 2^3 = kMaxHeads sets
+constexpr uint32_t kWideLevel = 3;         // the last level that any pool may open
+constexpr uint32_t kMaxLevel = 4;          // 2^4 = kMaxHeads sets
 constexpr uint32_t kRedirect = 0xfffffffeu;  // replace_head: use head set 0
 // surge trigger: warps that queued for one size's head lock during the life
 // of one head of set 0 (a grid of 1,024 warps can never reach it)
@@ -152,7 +154,7 @@ struct Config {
   uint32_t nib_words_sh;  // log2(words of nibbles per slab) = sb_sh - 7
   uint32_t set_words;     // ceil(nsbs / 32)
   uint32_t sum_words;     // ceil(set_words / 32)
-  uint32_t nheads;        // head slabs per size, a power of two <= kMaxHeads
+  uint32_t nheads;        // head slabs per size, a power of two <= kMaxFixedHeads
   uint32_t growth;        // 1: slabs are backed on demand (ha_grow_c)
   uint32_t surge;         // 1: head sets 1.. open under contention (nheads == 1 only)
   uint32_t spec_mask;     // bit s: size s adds its slab count with the reservation

@@ -110,16 +110,16 @@ bool g_nheads_set = false;  // ha_set_heads_c was called
 
 // Head slabs per size for an init.  A program written against halloc.h alone
 // cannot call ha_set_heads_c; HALLOC_HEADS in its environment (a power of
-// two up to kMaxHeads) sets the same knob.  An ha_set_heads_c call wins.
+// two up to kMaxFixedHeads) sets the same knob.  An ha_set_heads_c call wins.
 uint32_t heads_for_init() {
   if (g_nheads_set) return g_nheads;
   const char *e = getenv("HALLOC_HEADS");
   if (!e || !*e) return g_nheads;
   char *end = nullptr;
   const unsigned long v = strtoul(e, &end, 10);
-  if (*end || v == 0 || v > ha::kMaxHeads || (v & (v - 1))) {
+  if (*end || v == 0 || v > ha::kMaxFixedHeads || (v & (v - 1))) {
     fprintf(stderr, "halloc-b200: HALLOC_HEADS=%s ignored (a power of two from 1 to %u)\n", e,
-            (unsigned)ha::kMaxHeads);
+            (unsigned)ha::kMaxFixedHeads);
     return g_nheads;
   }
   return (uint32_t)v;
@@ -956,7 +956,7 @@ extern "C" int ha_dump_state_c(const ha_state_dump_t *d) {
 }
 
 extern "C" int ha_set_heads_c(uint32_t nheads) {
-  if (nheads == 0 || nheads > ha::kMaxHeads || (nheads & (nheads - 1))) return HA_EINVAL;
+  if (nheads == 0 || nheads > ha::kMaxFixedHeads || (nheads & (nheads - 1))) return HA_EINVAL;
   g_nheads = nheads;
   g_nheads_set = true;
   return HA_OK;
