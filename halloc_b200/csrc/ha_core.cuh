@@ -631,17 +631,19 @@ __device__ __noinline__ uint32_t find_slab(uint32_t sid) {
 }
 
 // Writes a surge level into size sid's set-0 head word, whose slab a warp may
-// be exchanging meanwhile (replace_head); true if the level was another.
+// be exchanging meanwhile (replace_head); true if the level was another.  Every
+// failed try is a head change of another warp; after 1,024 the level stays.
 __device__ __forceinline__ bool set_level(uint32_t sid, uint32_t level) {
   uint32_t w = ld_relaxed(&g_st.head[sid]);
-  for (;;) {
-    if (head_level(w) == level) return false;
+  for (uint32_t i = 0; i < 1024 && head_level(w) != level; i++) {
     const uint32_t seen = atom_cas(&g_st.head[sid], w, head_word(head_slab(w), level));
-    if (seen == w) break;
+    if (seen == w) {
+      st_relaxed(&g_st.level[sid], level);
+      return true;
+    }
     w = seen;
   }
-  st_relaxed(&g_st.level[sid], level);
-  return true;
+  return false;
 }
 
 // Whether any surge set of size sid holds a head or a prefetched slab (also
@@ -915,10 +917,10 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs, uint32_t crossed, boo
       after_change(hs, seen, wnew, judge, group);
       return next;
     }
+    // changed or closed meanwhile, or only its level changed: a caller still
+    // without a block comes again
     hand_back(hs, next);
     const uint32_t now = head_slab(was);
-    if (now != kNone && now != seen) return now;
-    // closed meanwhile, or only the level changed: the caller comes again
     return now == kNone ? none : now;
   }
   if (held == 0 && try_lock(hlock)) {
