@@ -77,7 +77,8 @@ def test_graph_degrees(torch_cuda, n, degrees):
         assert st["used_chunks"] == 0 and st["status"] == 0
 
 
-@pytest.mark.parametrize("n,ncells", [(1, 1), (31, 1), (129, 1), (2000, 1), (1000, 8), (5001, 3)])
+@pytest.mark.parametrize("n,ncells", [(1, 1), (31, 1), (129, 1), (2000, 1), (1000, 8), (5001, 3),
+                                      (1000, 41), (300000, 41), (999, 64)])
 def test_grid_lists(torch_cuda, n, ncells):
     import halloc_b200 as H
     from halloc_b200.workloads import sample_points
