@@ -216,17 +216,22 @@ __global__ void __launch_bounds__(kGridBlock) ha_grid_free_k(uint32_t ncells3, P
 // pairs of 0 to 31 characters, word by word -> by pairs: concatenation 83 ->
 // 73 us, check (byte by byte) 47 -> 28 us, allocation 49 -> 43 us.
 //
-// The second word of a pair may lie 8 bytes past a string's block: only the
-// 24-byte blocks hold an odd number of words, and a slab of 24-byte chunks ends
-// with at least 64 bytes that belong to no block; blocks of CUDA's heap are
-// 16-byte aligned, so their pairs never leave a 16-byte granule.  What such
-// a word holds is not used.
+// Every pair is one 16-byte granule: a string that starts in the upper half of
+// one (24-byte blocks do) is read a single word first.  So no load leaves the
+// granules that hold a byte of the string, wherever the string lies; what a
+// pair holds past its string is not used.
 
 constexpr uint64_t kSpaces = 0x2020202020202020ull;
 
 struct Pair {
   uint64_t x, y;
 };
+// words from p to the end of its 16-byte granule: 1 or 2
+__device__ __forceinline__ uint32_t words_at(const uint64_t *p) {
+  return 2 - (((uintptr_t)p >> 3) & 1u);
+}
+// the words_at(p) words from p on; the second of one word reads as all ones,
+// which holds no zero byte
 __device__ __forceinline__ Pair load_pair(const uint64_t *p) {
   Pair v;
   if (((uintptr_t)p & 15u) == 0) {
@@ -235,7 +240,7 @@ __device__ __forceinline__ Pair load_pair(const uint64_t *p) {
     v.y = q.y;
   } else {
     v.x = p[0];
-    v.y = p[1];
+    v.y = ~0ull;
   }
   return v;
 }
@@ -310,12 +315,14 @@ __global__ void ha_strings_concat_k(uint32_t n, char **c, char *const *a, char *
   }
   uint32_t la = 0, lb = 0;
   bool enda = false, endb = false;
-  for (uint32_t k = 0; !enda || !endb; k += 2) {
+  for (uint32_t i = 0, j = 0; !enda || !endb;) {
     Pair va = {0, 0}, vb = {0, 0};
-    if (!enda) va = load_pair(sa + k);
-    if (!endb) vb = load_pair(sb + k);
-    if (!enda) enda = ends_in(va, 8 * k, la);
-    if (!endb) endb = ends_in(vb, 8 * k, lb);
+    if (!enda) va = load_pair(sa + i);
+    if (!endb) vb = load_pair(sb + j);
+    if (!enda) enda = ends_in(va, 8 * i, la);
+    if (!endb) endb = ends_in(vb, 8 * j, lb);
+    i += words_at(sa + i);
+    j += words_at(sb + j);
   }
   const uint32_t lc = la + lb;
   const uint32_t cwords = lc / 8 + 1;
@@ -362,27 +369,35 @@ __global__ void ha_strings_free_k(uint32_t n, char **strs) {
 
 // counts strings that are not la[i] + lb[i] spaces followed by a zero byte
 // (by pairs of words; a pair is read only once all before it are spaces, so
-// the string reaches at least to its start)
+// the string reaches at least to its start).  Strings may lie anywhere: one
+// that does not start on a word is read byte by byte.
 __global__ void ha_strings_check_k(uint32_t n, char *const *c, const int *la, const int *lb,
                                    unsigned long long *bad) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint64_t *s = reinterpret_cast<const uint64_t *>(c[i]);
   const uint32_t want = (uint32_t)(la[i] + lb[i]);
-  const uint32_t full = want / 8, z = want % 8;  // the zero byte: byte z of word `full`
-  const uint64_t mask = z == 7 ? ~0ull : (1ull << (8 * (z + 1))) - 1;
-  const uint64_t tail = z ? kSpaces >> (8 * (8 - z)) : 0ull;
   bool ok = s != nullptr;
-  uint32_t k = 0;
-  for (; ok && k + 1 < full; k += 2) {
-    const Pair v = load_pair(s + k);
-    ok = v.x == kSpaces && v.y == kSpaces;
-  }
-  if (ok && k < full) {  // one whole word left, then the last
-    const Pair v = load_pair(s + k);
-    ok = v.x == kSpaces && (v.y & mask) == tail;
+  if (((uintptr_t)s & 7u) != 0) {
+    const char *t = c[i];
+    for (uint32_t k = 0; ok && k < want; k++) ok = t[k] == ' ';
+    if (ok) ok = t[want] == 0;
   } else if (ok) {
-    ok = (s[k] & mask) == tail;
+    const uint32_t full = want / 8, z = want % 8;  // the zero byte: byte z of word `full`
+    const uint64_t mask = z == 7 ? ~0ull : (1ull << (8 * (z + 1))) - 1;
+    const uint64_t tail = z ? kSpaces >> (8 * (8 - z)) : 0ull;
+    uint32_t k = 0;
+    if (full && words_at(s) == 1) ok = s[k++] == kSpaces;
+    for (; ok && k + 1 < full; k += 2) {
+      const Pair v = load_pair(s + k);
+      ok = v.x == kSpaces && v.y == kSpaces;
+    }
+    if (ok && k < full) {  // one whole word left, then the last, in one granule
+      const Pair v = load_pair(s + k);
+      ok = v.x == kSpaces && (v.y & mask) == tail;
+    } else if (ok) {
+      ok = (s[k] & mask) == tail;
+    }
   }
   if (!ok) atomicAdd(bad, 1ull);
 }

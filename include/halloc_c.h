@@ -382,14 +382,17 @@ int ha_grid_free_c(uint32_t ncells, void **grid, int pre_nodes, void *stream);
    becomes lens[i] spaces and a zero byte in a block from hamalloc
    (strs: device, n pointers); concat makes c[i] = a[i] followed by b[i] in a
    new block; free releases and clears every string.  Strings are read and
-   written as 64-bit words.  nfail (device, accumulated): NULL blocks. */
+   written as 64-bit words, so those given to concat start on an 8-byte
+   boundary; no read leaves the aligned 16-byte granules that hold a byte of
+   a string.  nfail (device, accumulated): NULL blocks. */
 int ha_strings_alloc_c(uint32_t n, const int *lens, char **strs, uint64_t *nfail,
                        void *stream);
 int ha_strings_concat_c(uint32_t n, char **c, char *const *a, char *const *b,
                         uint64_t *nfail, void *stream);
 int ha_strings_free_c(uint32_t n, char **strs, void *stream);
 /* bad (device, accumulated): strings c[i] that are not la[i] + lb[i] spaces
-   and a zero byte. */
+   and a zero byte.  A string may start at any address, from hamalloc or
+   not; the reads are those of concat. */
 int ha_strings_check_c(uint32_t n, char *const *c, const int *la, const int *lb,
                        uint64_t *bad, void *stream);
 
