@@ -302,6 +302,9 @@ __global__ void __launch_bounds__(1024) ha_serve_k(ServeParams P) {
         if (++j.steps >= j.life) draining = true;
       }
     }
+    // the links and values that other lanes wrote above are read below, in
+    // this step or a later one: shuffles and votes order no memory
+    __syncwarp();
     // drain: every draining job walks up to P.depth nodes of its list at a
     // time, then the warp frees them
     for (uint32_t left = kDrainPerStep;
