@@ -26,6 +26,7 @@
 #include <stdint.h>
 
 #include "ha_types.h"
+#include "ha_ptx.cuh"
 #include "ha_stamp.cuh"
 
 namespace ha {
@@ -38,149 +39,6 @@ extern __device__ Class g_cls[kNSizes];
 // fastmod magics per size class: nchunks (x, y = low, high word), hash step (z, w)
 extern __device__ uint4 g_mod[kNSizes];
 extern __device__ State g_st;
-
-// ---------------------------------------------------------------------------
-// PTX helpers: explicit scope and ordering
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t lane_id() {
-  uint32_t l;
-  asm("mov.u32 %0, %%laneid;" : "=r"(l));
-  return l;
-}
-__device__ __forceinline__ uint32_t lanemask_lt() {
-  uint32_t m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
-// Whether this lane is the first of group `grp` it belongs to (three times
-// quicker than comparing its id with the group's lowest set bit).
-__device__ __forceinline__ bool first_of(uint32_t grp) { return (grp & lanemask_lt()) == 0; }
-__device__ __forceinline__ uint32_t sm_id() {
-  uint32_t v;
-  asm("mov.u32 %0, %%smid;" : "=r"(v));
-  return v;
-}
-__device__ __forceinline__ uint64_t globaltimer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-// may return a value that this SM read earlier in the same launch
-__device__ __forceinline__ uint32_t ld_cached(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v) {
-  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t atom_add(uint32_t *p, uint32_t v) {
-  uint32_t o;
-  asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], %2;"
-               : "=r"(o) : "l"(p), "r"(v));
-  return o;
-}
-__device__ __forceinline__ uint32_t atom_or(uint32_t *p, uint32_t v) {
-  uint32_t o;
-  asm volatile("atom.relaxed.gpu.global.or.b32 %0, [%1], %2;"
-               : "=r"(o) : "l"(p), "r"(v));
-  return o;
-}
-__device__ __forceinline__ uint32_t atom_and(uint32_t *p, uint32_t v) {
-  uint32_t o;
-  asm volatile("atom.relaxed.gpu.global.and.b32 %0, [%1], %2;"
-               : "=r"(o) : "l"(p), "r"(v));
-  return o;
-}
-__device__ __forceinline__ void red_add(uint32_t *p, uint32_t v) {
-  asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v));
-}
-__device__ __forceinline__ void red_or(uint32_t *p, uint32_t v) {
-  asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(v));
-}
-__device__ __forceinline__ void red_and(uint32_t *p, uint32_t v) {
-  asm volatile("red.relaxed.gpu.global.and.b32 [%0], %1;" ::"l"(p), "r"(v));
-}
-__device__ __forceinline__ uint32_t atom_cas(uint32_t *p, uint32_t expect, uint32_t v) {
-  uint32_t o;
-  asm volatile("atom.acq_rel.gpu.global.cas.b32 %0, [%1], %2, %3;"
-               : "=r"(o) : "l"(p), "r"(expect), "r"(v) : "memory");
-  return o;
-}
-__device__ __forceinline__ uint32_t atom_exch(uint32_t *p, uint32_t v) {
-  uint32_t o;
-  asm volatile("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;"
-               : "=r"(o) : "l"(p), "r"(v) : "memory");
-  return o;
-}
-__device__ __forceinline__ void fence_acq_rel() {
-  asm volatile("fence.acq_rel.gpu;" ::: "memory");
-}
-
-// Slab metadata accesses (bit arrays, size nibbles, slab counters) carry an
-// L2 evict-last cache policy, so that the metadata of the slabs in use stays
-// in L2 while payload streams through it -- for every kernel that calls
-// hamalloc / hafree, not only those launched on a stream with an access-
-// policy window (ha_l2_persist_c).  Build with -DHA_L2_HINTS=0 for plain
-// accesses.  (halloc's analogue: cudaFuncCachePreferL1 and ld.global.ca
-// metadata loads, src/halloc.cu:279, src/utils.h:141-157.)
-#ifndef HA_L2_HINTS
-#define HA_L2_HINTS 1
-#endif
-#if HA_L2_HINTS
-__device__ __forceinline__ uint64_t meta_policy() {
-  uint64_t p;
-  asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ uint32_t ld_meta(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.L2::cache_hint.u32 %0, [%1], %2;"
-               : "=r"(v) : "l"(p), "l"(meta_policy()));
-  return v;
-}
-__device__ __forceinline__ uint32_t atom_add_meta(uint32_t *p, uint32_t v) {
-  uint32_t o;
-  asm volatile("atom.relaxed.gpu.global.add.L2::cache_hint.u32 %0, [%1], %2, %3;"
-               : "=r"(o) : "l"(p), "r"(v), "l"(meta_policy()));
-  return o;
-}
-__device__ __forceinline__ uint32_t atom_or_meta(uint32_t *p, uint32_t v) {
-  uint32_t o;
-  asm volatile("atom.relaxed.gpu.global.or.L2::cache_hint.b32 %0, [%1], %2, %3;"
-               : "=r"(o) : "l"(p), "r"(v), "l"(meta_policy()));
-  return o;
-}
-__device__ __forceinline__ uint32_t atom_and_meta(uint32_t *p, uint32_t v) {
-  uint32_t o;
-  asm volatile("atom.relaxed.gpu.global.and.L2::cache_hint.b32 %0, [%1], %2, %3;"
-               : "=r"(o) : "l"(p), "r"(v), "l"(meta_policy()));
-  return o;
-}
-__device__ __forceinline__ void red_or_meta(uint32_t *p, uint32_t v) {
-  asm volatile("red.relaxed.gpu.global.or.L2::cache_hint.b32 [%0], %1, %2;"
-               ::"l"(p), "r"(v), "l"(meta_policy()));
-}
-__device__ __forceinline__ void red_and_meta(uint32_t *p, uint32_t v) {
-  asm volatile("red.relaxed.gpu.global.and.L2::cache_hint.b32 [%0], %1, %2;"
-               ::"l"(p), "r"(v), "l"(meta_policy()));
-}
-#else
-__device__ __forceinline__ uint32_t ld_meta(const uint32_t *p) { return ld_relaxed(p); }
-__device__ __forceinline__ uint32_t atom_add_meta(uint32_t *p, uint32_t v) { return atom_add(p, v); }
-__device__ __forceinline__ uint32_t atom_or_meta(uint32_t *p, uint32_t v) { return atom_or(p, v); }
-__device__ __forceinline__ uint32_t atom_and_meta(uint32_t *p, uint32_t v) { return atom_and(p, v); }
-__device__ __forceinline__ void red_or_meta(uint32_t *p, uint32_t v) { red_or(p, v); }
-__device__ __forceinline__ void red_and_meta(uint32_t *p, uint32_t v) { red_and(p, v); }
-#endif
 
 // ---------------------------------------------------------------------------
 // status, bounded waits, locks
@@ -515,6 +373,32 @@ __device__ __noinline__ void retire(uint32_t sb) {
     set_put(kSetBusy + sid, sb);
 }
 
+// A change of head slot hs is marked (State::changing) from before its warp
+// takes a slab out of the slot or the sets until that slab is the head, the
+// prefetched slab or filed: a warp that found nothing and then reads no marks
+// finds whatever was on its way (search_on).
+__device__ __forceinline__ void mark_change(uint32_t hs) { red_add(&g_st.changing[hs], 1u); }
+
+// Takes head slot hs's prefetched slab (kNone if there is none).  The fence
+// orders the caller's mark before this and every later taking, and is the
+// exchange's release, too.
+__device__ __forceinline__ uint32_t take_prefetched(uint32_t hs) {
+  fence_acq_rel();
+  return atom_exch_acquire(&g_st.cached[hs], kNone);
+}
+
+// Ends a marked change of head slot hs: the slab sb that the caller still holds
+// (kNone: none) becomes the slot's prefetched slab or, when another landed
+// there first, is filed again.
+__device__ __noinline__ void settle(uint32_t hs, uint32_t sb) {
+  if (sb != kNone && atom_cas(&g_st.cached[hs], kNone, sb) != kNone &&
+      lock(&g_st.sb_lock[sb])) {
+    detach(sb);
+    unlock(&g_st.sb_lock[sb]);
+  }
+  red_add_release(&g_st.changing[hs], 0u - 1u);
+}
+
 // Closes surge head set hs (set 1 or above): its head and its prefetched slab
 // are retired.  Unless `force`, only while the size's set-0 head word says
 // the set is closed (a set opened again meanwhile keeps its head).
@@ -527,8 +411,8 @@ __device__ __noinline__ void retire_set(uint32_t hs, bool force) {
     return;
   }
   const uint32_t old = head_slab(atom_exch(&g_st.head[hs], kSlabField));
-  cuda::atomic_ref<uint32_t, cuda::thread_scope_device> cached(g_st.cached[hs]);
-  const uint32_t pre = cached.exchange(kNone, cuda::memory_order_acq_rel);
+  mark_change(hs);
+  const uint32_t pre = take_prefetched(hs);
   unlock(hlock);
   if (old != kNone && lock(&g_st.sb_lock[old])) {
     retire(old);
@@ -538,6 +422,7 @@ __device__ __noinline__ void retire_set(uint32_t hs, bool force) {
     retire(pre);
     unlock(&g_st.sb_lock[pre]);
   }
+  settle(hs, kNone);
 }
 
 // Picks the next head slab for a size: roomy slabs of the size, sparse slabs
@@ -683,19 +568,6 @@ __device__ __noinline__ bool close_other_surges(uint32_t own) {
   return any;
 }
 
-// Hands a slab taken for head slot hs back to hs's prefetch slot, or, when
-// another prefetch landed there first, files it again.
-__device__ __noinline__ void hand_back(uint32_t hs, uint32_t sb) {
-  cuda::atomic_ref<uint32_t, cuda::thread_scope_device> cached(g_st.cached[hs]);
-  uint32_t expect = kNone;
-  if (!cached.compare_exchange_strong(expect, sb, cuda::memory_order_acq_rel)) {
-    if (lock(&g_st.sb_lock[sb])) {
-      detach(sb);
-      unlock(&g_st.sb_lock[sb]);
-    }
-  }
-}
-
 // Whether a size may open surge level `level`: more heads hold more partly
 // filled slabs, so only while a quarter of the pool is free.  The topmost
 // level, whose heads and prefetched slabs are 32, opens only in pools of at
@@ -810,7 +682,8 @@ __device__ __forceinline__ uint32_t judge_level(uint32_t sid, uint32_t level, bo
 
 // What follows a change of head slot hs from slab `old` to `next`: the old
 // head is filed, the surge level judged (set 0), and the next slab
-// prefetched, the reference's steps in the reference's order.
+// prefetched, the reference's steps in the reference's order.  Ends the
+// caller's mark.
 __device__ __noinline__ void after_change(uint32_t hs, uint32_t old, uint32_t wnew, bool judge,
                                           bool group) {
   const uint32_t sid = hs % kNSizes;
@@ -819,8 +692,7 @@ __device__ __noinline__ void after_change(uint32_t hs, uint32_t old, uint32_t wn
     detach(old);
     unlock(&g_st.sb_lock[old]);
   }
-  const uint32_t pre = find_slab(sid);
-  if (pre != kNone) hand_back(hs, pre);
+  settle(hs, find_slab(sid));
   if (judge) {
     const uint32_t level = head_level(wnew), nlevel = judge_level(sid, level, group);
     // given up when the head changed meanwhile: that change is judged itself
@@ -831,6 +703,63 @@ __device__ __noinline__ void after_change(uint32_t hs, uint32_t old, uint32_t wn
       // a level closed: retire the heads of its sets
       for (uint32_t k = 1u << nlevel; k < (1u << level); k++)
         retire_set(k * kNSizes + sid, false);
+    }
+  }
+}
+
+// A slab for head slot hs after a search (begun at `epoch`) found none; the
+// caller holds the slot's lock and has marked a change of it.  For head set 0
+// with surge sets on (`judge`) the size's surge sets are closed, which files
+// their heads and prefetched slabs where a search finds them (`closed`), then
+// those of other sizes.  kNone means that no slab was left for the size: in one
+// pass after the last search (begun at `epoch`) no head of a surge set, no
+// prefetched slab, no change under way (which may hold a slab that is in no set,
+// and is waited for) and no newly filed slab was seen.  `moved`: another warp
+// changed the head `cur` meanwhile.  No warp waits here for this one: those under
+// way take no lock of head set 0 (a warp that has to wait for it ends its change
+// first), and head sets 1 and above do not come here.
+__device__ __noinline__ uint32_t search_on(uint32_t hs, uint32_t cur, bool judge, uint32_t &epoch,
+                                           bool &closed, bool &moved) {
+  const uint32_t sid = hs % kNSizes;
+  Deadline dl;
+  bool others = judge;  // the surge sets of other sizes are still to be closed
+  for (uint32_t quiet = 0;;) {
+    if (judge && surge_slabs_held(sid)) {
+      if (set_level(sid, 0)) red_add(&g_st.n_surge_changes, 1);
+      for (uint32_t k = 1; k < kMaxHeads; k++) retire_set(k * kNSizes + sid, true);
+      closed = true;
+    }
+    fence_acq_rel();  // what was not found, then the marks
+    // (fixed head sets keep their slabs to themselves)
+    bool under_way = ld_relaxed(&g_st.changing[hs]) > 1;  // one mark is the caller's
+    for (uint32_t k = 1; k < kMaxHeads && judge; k++)
+      under_way |= ld_relaxed(&g_st.changing[k * kNSizes + sid]) != 0;
+    fence_acq_rel();  // the marks, then where a change that has ended left its slab
+    if (head_slab(ld_relaxed(&g_st.head[hs])) != cur) {
+      moved = true;
+      return kNone;
+    }
+    if (ld_relaxed(&g_st.cached[hs]) != kNone) {
+      const uint32_t sb = take_prefetched(hs);
+      if (sb != kNone) return sb;
+    }
+    const uint32_t now = ld_relaxed(&g_st.set_epoch);
+    const bool filed = now != epoch;
+    if (filed) {
+      epoch = now;
+      const uint32_t sb = find_slab(sid);
+      if (sb != kNone) return sb;
+    }
+    if (others) {
+      others = false;
+      close_other_surges(sid);
+    } else if (!under_way && (!filed || ++quiet == 64)) {
+      return kNone;  // (other sizes may file slabs at any rate)
+    } else if (dl.expired()) {
+      raise_status(HA_ST_TIMEOUT);
+      return kNone;
+    } else if (under_way) {
+      dl.backoff();
     }
   }
 }
@@ -852,7 +781,7 @@ __device__ __noinline__ void after_change(uint32_t hs, uint32_t old, uint32_t wn
 // that loses the race for it waits (bounded) until the head changes or the
 // lock is released.  Filing the old head and prefetching follow the change; a
 // single thread still performs the reference's steps in the reference's order.
-// Two prefetches can overlap: the loser hands its slab back.
+// Two prefetches can overlap: the loser's slab is filed again.
 //
 // Surge sets (c_cfg.surge): when thousands of warps queue for one size's
 // head (a grid far larger than its head's free space), set 0's changes open
@@ -872,41 +801,52 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs, uint32_t crossed, boo
   const uint32_t none = surge_set ? kRedirect : kNone;  // "no head" answer
   uint32_t *head = &g_st.head[hs];
   uint32_t *hlock = &g_st.head_lock[hs * kTicketStride];
-  uint32_t *cached = &g_st.cached[hs];
   const uint32_t busy = load_class(sid).busy;
   // One round trip for the head, the memo below, the lock word, the prefetched
   // slab and (surge sets) set 0's head word.
   const uint32_t wseen = ld_relaxed(head);
-  const uint32_t epoch = ld_relaxed(&g_st.set_epoch);
+  uint32_t epoch = ld_relaxed(&g_st.set_epoch);
   const uint32_t memo = ld_relaxed(&g_st.no_slab[hs]);
   const uint32_t held = ld_relaxed(hlock);
   const uint32_t w0 = surge_set ? ld_relaxed(&g_st.head[sid]) : 0u;
-  const uint32_t ready = ld_relaxed(cached);
-  uint32_t next = crossed != kNone ? atom_exch(cached, kNone) : kNone;
+  const uint32_t ready = ld_relaxed(&g_st.cached[hs]);
+  const uint32_t under_way = ld_relaxed(&g_st.changing[hs]);
+  // from the mark on, every way out settles
+  bool marked = false;
+  uint32_t next = kNone;
+  if (crossed != kNone) {
+    mark_change(hs);
+    marked = true;
+    next = take_prefetched(hs);
+  }
   const uint32_t seen = head_slab(wseen);
   if (surge_set && set >= (1u << head_level(w0))) {
     if (next != kNone && lock(&g_st.sb_lock[next])) {
       retire(next);
       unlock(&g_st.sb_lock[next]);
     }
+    if (marked) settle(hs, kNone);
     return kRedirect;
   }
   if (crossed != kNone && seen != crossed) {  // changed already
-    if (next != kNone) hand_back(hs, next);
+    settle(hs, next);
     return seen == kNone ? none : seen;
   }
   if (crossed == kNone) {
     // A failed search leaves every set it looked at empty, so until a slab is
     // filed somewhere (set_epoch moves) another search would fail the same
-    // way: answer at once instead of queueing for the lock to search again.
-    if (memo == epoch + 1u && (seen == kNone || used_of(seen) >= busy)) return none;
+    // way: answer at once instead of queueing for the lock to search again,
+    // unless a slab lies prefetched or (where the answer is NULL) a change is
+    // under way that may bring one.
+    const bool dry = ready == kNone && (surge_set || under_way == 0);
+    if (memo == epoch + 1u && dry && (seen == kNone || used_of(seen) >= busy)) return none;
     if (seen != kNone) {
-      const uint32_t n_seen = used_of(seen);
-      if (ready != kNone) next = atom_exch(cached, kNone);
-      if (n_seen < busy) {
-        // not busy after all (the reference's re-check): hand the slab back
-        if (next != kNone) hand_back(hs, next);
-        return seen;
+      // not busy after all (the reference's re-check)
+      if (used_of(seen) < busy) return seen;
+      if (ready != kNone) {
+        mark_change(hs);
+        marked = true;
+        next = take_prefetched(hs);
       }
     }
   }
@@ -919,16 +859,18 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs, uint32_t crossed, boo
     }
     // changed or closed meanwhile, or only its level changed: a caller still
     // without a block comes again
-    hand_back(hs, next);
+    settle(hs, next);
     const uint32_t now = head_slab(was);
     return now == kNone ? none : now;
   }
   if (held == 0 && try_lock(hlock)) {
     // Under the lock, one round trip again: the head and set 0's word (surge
     // sets) as they are now and a slab prefetched meanwhile.
+    if (!marked) mark_change(hs);
     const uint32_t wcur = ld_relaxed(head);
+    epoch = ld_relaxed(&g_st.set_epoch);
     const uint32_t w0now = surge_set ? ld_relaxed(&g_st.head[sid]) : 0u;
-    next = atom_exch(cached, kNone);
+    next = take_prefetched(hs);
     const uint32_t cur = head_slab(wcur);
     if (surge_set && set >= (1u << head_level(w0now))) {
       // the set closed while this warp came for its lock
@@ -937,36 +879,36 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs, uint32_t crossed, boo
         retire(next);
         unlock(&g_st.sb_lock[next]);
       }
+      settle(hs, kNone);
       return kRedirect;
     }
     if (cur != seen && cur != kNone && used_of(cur) < busy) {
-      if (next != kNone) hand_back(hs, next);
       unlock(hlock);
+      settle(hs, next);
       return cur;
     }
     const uint32_t level = judge ? head_level(wcur) : 0u;
     uint32_t nlevel = level;
     if (next == kNone) next = find_slab(sid);
-    if (next == kNone && judge && surge_slabs_held(sid)) {
-      // short of slabs while surge sets hold heads: close them all, which
-      // files their heads and prefetched slabs where this search finds them
-      for (uint32_t k = 1; k < kMaxHeads; k++) retire_set(k * kNSizes + sid, true);
-      nlevel = 0;
-      next = find_slab(sid);
+    if (next == kNone && !surge_set) {
+      bool closed = false, moved = false;
+      next = search_on(hs, cur, judge, epoch, closed, moved);
+      if (closed) nlevel = 0;
+      if (moved) {
+        unlock(hlock);
+        settle(hs, kNone);
+        const uint32_t now = head_slab(ld_relaxed(head));
+        return now == kNone ? none : now;
+      }
     }
-    if (next == kNone && judge && close_other_surges(sid)) next = find_slab(sid);
     if (next == kNone) {
       st_relaxed(&g_st.no_slab[hs], epoch + 1u);
-      if (nlevel != level) set_level(sid, nlevel);
       unlock(hlock);
+      settle(hs, kNone);
       return none;
     }
     const uint32_t wnew = head_word(next, nlevel);
     const uint32_t was = head_slab(atom_exch(head, wnew));
-    if (nlevel != level) {
-      st_relaxed(&g_st.level[sid], nlevel);
-      red_add(&g_st.n_surge_changes, 1);
-    }
     unlock(hlock);
     if (was != cur && was != kNone) {
       // another warp's change came in between: its head may not be busy yet
@@ -980,6 +922,7 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs, uint32_t crossed, boo
     }
     return next;
   }
+  if (marked) settle(hs, kNone);  // nothing held while it waits
   // Every warp that found the head busy and no slab prefetched waits here,
   // thousands at once when a grid storms one size.  Their polls all go to the
   // sectors of the head and lock words, which the lock holder must write to
@@ -1426,14 +1369,6 @@ __device__ __forceinline__ void *malloc_small(uint32_t nbytes) {
   }
   HA_STAMP(kStMallocOut, (uint32_t)(uintptr_t)p);
   return p;
-}
-
-__device__ __forceinline__ Desc ld_desc(const Desc *p) {
-  Desc d;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(d.size_id), "=r"(d.chunk_id), "=r"(d.is_head), "=r"(d.chunk_enc)
-               : "l"(p));
-  return d;
 }
 
 // Whether a count of n0 chunks lowered by n crosses a threshold of size sid

@@ -178,6 +178,9 @@ struct State {
   uint32_t head_lock[kMaxHeads * kNSizes * kTicketStride];
   alignas(128) uint32_t head[kMaxHeads * kNSizes];
   uint32_t cached[kMaxHeads * kNSizes];
+  // per head slot: changes of it that are under way -- warps that may hold a
+  // slab which is in no set and no slot
+  alignas(128) uint32_t changing[kMaxHeads * kNSizes];
   // per size: a copy of the surge level, for loads that L1 may serve
   alignas(128) uint32_t level[kTicketStride];
   alignas(128) uint32_t status;
