@@ -320,14 +320,24 @@ __device__ __forceinline__ void count_down(uint32_t mask, uint32_t sb, uint32_t 
 // lock.  The first comparison uses the ROOMY threshold of the slab's size and
 // the next two read the size-table entry whose index equals the chunk id;
 // both are the reference's rules (halloc src/slab.cuh:227-255) and are kept
-// for identical set contents.
+// for identical set contents.  The reference leaves a slab above the roomy
+// threshold out of every set, as its head is busy when it is detached.  Here
+// other warps' frees, or early counts that were taken back, may have brought
+// the head under the busy threshold after its change was begun; the free that
+// crossed the threshold did not file it, as it was a head then, so it is filed
+// here (a lone thread never detaches such a head).
 __device__ __noinline__ void detach(uint32_t sb) {
   Desc *d = &g_st.desc[desc_index(sb)];
   st_relaxed(&d->is_head, 0);
   uint32_t before = atom_add(ctr_of(sb), 0u - kHeadFlag);
   uint32_t n = before >> kCntShift;
   uint32_t sid = ld_relaxed(&d->size_id);
-  if (sid >= kNSizes || n > load_class(sid).roomy) return;
+  if (sid >= kNSizes) return;
+  const Class c = load_class(sid);
+  if (n > c.roomy) {
+    if (n < c.busy) set_put(kSetBusy + sid, sb);
+    return;
+  }
   uint32_t cid = ld_relaxed(&d->chunk_id);
   if (n == 0) {
     try_release(sb, cid, true);
@@ -393,7 +403,7 @@ __device__ __forceinline__ uint32_t take_prefetched(uint32_t hs) {
 __device__ __noinline__ void settle(uint32_t hs, uint32_t sb) {
   if (sb != kNone && atom_cas(&g_st.cached[hs], kNone, sb) != kNone &&
       lock(&g_st.sb_lock[sb])) {
-    detach(sb);
+    retire(sb);  // filled to whatever the set held that it came from
     unlock(&g_st.sb_lock[sb]);
   }
   red_add_release(&g_st.changing[hs], 0u - 1u);

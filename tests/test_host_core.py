@@ -76,3 +76,55 @@ def test_a_null_leaves_no_slab_unused(core, size, lanes, surge):
         assert core.head(sid)["prefetched"] == NONE, seed
         used = [core.slab(sb)["used"] for sb in range(nsbs)]
         assert min(used) >= busy - nwarps * lanes * ncib, (seed, used)
+
+
+def churn(rng, nops, lanes, sizes, p_free, keep=0.0):
+    """A warp's random allocations and frees; what it holds at the end it frees
+    but for the share `keep`."""
+    ops, held = [], []
+    for _ in range(nops):
+        if held and rng.random() < p_free:
+            ops.append([-held.pop(rng.integers(len(held))) - 1] * lanes)
+        else:
+            held.append(len(ops))
+            ops.append(list(rng.choice(sizes, lanes)))
+    ops += [[-k - 1] * lanes for k in held if rng.random() >= keep]
+    return np.array(ops)
+
+
+def assert_quiescent(core, res, seed):
+    """No block handed out twice, the counts those of the blocks held, and every
+    slab where it belongs: a head, a prefetched slab or in a set."""
+    held = np.concatenate([r[r >= 0] for r in res])
+    assert len(np.unique(held)) == len(held), seed
+    owned = {core.head(s, k)[w] for s in range(16) for k in range(16)
+             for w in ("slab", "prefetched")}
+    for sb in range(core.nsbs):
+        d = core.slab(sb)
+        blocks = int(((held >> core.sb_sh) == sb).sum())
+        ncib = int(core.cls[d["size_id"], 3]) if d["size_id"] != NONE else 0
+        assert d["is_head"] == d["head_flag"] == (sb in owned), (seed, sb, d)
+        assert (d["used"] == 0) == (blocks == 0), (seed, sb, d)
+        if d["is_head"] or d["size_id"] == NONE:
+            continue
+        # A head that is detached with exactly its busy threshold in use is in no
+        # set until it is roomy (the reference's rule); blocks of several chunks
+        # never add up to a threshold that is odd.
+        busy = int(core.cls[d["size_id"], 7])
+        if ncib > 1 and busy % 2 and d["used"] < busy:
+            assert d["nsets"] > 0, (seed, sb, d)
+
+
+@pytest.mark.parametrize("surge", [0, 1])
+@pytest.mark.parametrize("sizes,lanes", [([2048], 1), ([2048], 4), ([1024, 2048], 2),
+                                         ([512, 768, 2048], 4)])
+def test_a_slab_with_room_is_in_a_set(core, sizes, lanes, surge):
+    """Warps allocate and free at random and hold half of what they have at the
+    end: frees race the changes of the heads that they free into."""
+    for seed in range(250):
+        rng = np.random.default_rng(seed)
+        core.init(int(rng.integers(4, 16)), surge=surge)
+        res = core.run([churn(rng, int(rng.integers(20, 120)), lanes, sizes, 0.4, 0.5)
+                        for _ in range(int(rng.integers(2, 12)))], seed)
+        assert core.status == 0, seed
+        assert_quiescent(core, res, seed)
