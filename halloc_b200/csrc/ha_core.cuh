@@ -525,20 +525,39 @@ __device__ __noinline__ uint32_t find_slab(uint32_t sid) {
   return kNone;
 }
 
+// Brings the copy of size sid's surge level up to date, after every change of
+// the level in set 0's head word.  Two changes may be copied in either order: a
+// warp copies again while the word shows another level than it copied, and
+// with a fence on either side of the copy the warp whose copy lands last sees
+// the last change.
+__device__ __forceinline__ void copy_level(uint32_t sid) {
+  uint32_t level = head_level(ld_relaxed(&g_st.head[sid]));
+  for (uint32_t i = 0; i < 1024; i++) {
+    fence_sc();
+    st_relaxed(&g_st.level[sid], level);
+    fence_sc();
+    const uint32_t now = head_level(ld_relaxed(&g_st.head[sid]));
+    if (now == level) return;
+    level = now;
+  }
+}
+
 // Writes a surge level into size sid's set-0 head word, whose slab a warp may
-// be exchanging meanwhile (replace_head); true if the level was another.  Every
+// be exchanging meanwhile (replace_head); whether it stands there now.  Every
 // failed try is a head change of another warp; after 1,024 the level stays.
 __device__ __forceinline__ bool set_level(uint32_t sid, uint32_t level) {
   uint32_t w = ld_relaxed(&g_st.head[sid]);
   for (uint32_t i = 0; i < 1024 && head_level(w) != level; i++) {
     const uint32_t seen = atom_cas(&g_st.head[sid], w, head_word(head_slab(w), level));
     if (seen == w) {
-      st_relaxed(&g_st.level[sid], level);
-      return true;
+      red_add(&g_st.n_surge_changes, 1);
+      w = head_word(head_slab(w), level);
+    } else {
+      w = seen;
     }
-    w = seen;
   }
-  return false;
+  copy_level(sid);
+  return head_level(w) == level;
 }
 
 // Whether any surge set of size sid holds a head or a prefetched slab (also
@@ -568,9 +587,8 @@ __device__ __noinline__ bool close_other_surges(uint32_t own) {
     uint32_t *hlock0 = &g_st.head_lock[sid * kTicketStride];
     bool closed = false;
     if (ld_relaxed(hlock0) == 0 && try_lock(hlock0)) {
-      if (set_level(sid, 0)) red_add(&g_st.n_surge_changes, 1);
+      closed = set_level(sid, 0);
       unlock(hlock0);
-      closed = true;
     }
     for (uint32_t k = 1; k < kMaxHeads; k++) retire_set(k * kNSizes + sid, !closed);
     any = true;
@@ -608,8 +626,8 @@ __device__ __forceinline__ void surge_open(uint32_t sid) {
   const uint32_t committed = ld_relaxed(&g_st.committed);
   if (head_slab(w) != kNone && room_for_level(level + 1, nfree, committed)) {
     if (atom_cas(head, w, head_word(head_slab(w), level + 1)) == w) {
-      st_relaxed(&g_st.level[sid], level + 1);
       red_add(&g_st.n_surge_changes, 1);
+      copy_level(sid);
     }
   }
   unlock(hlock);
@@ -708,8 +726,8 @@ __device__ __noinline__ void after_change(uint32_t hs, uint32_t old, uint32_t wn
     // given up when the head changed meanwhile: that change is judged itself
     if (nlevel != level &&
         atom_cas(&g_st.head[hs], wnew, head_word(head_slab(wnew), nlevel)) == wnew) {
-      st_relaxed(&g_st.level[sid], nlevel);
       red_add(&g_st.n_surge_changes, 1);
+      copy_level(sid);
       // a level closed: retire the heads of its sets
       for (uint32_t k = 1u << nlevel; k < (1u << level); k++)
         retire_set(k * kNSizes + sid, false);
@@ -735,7 +753,7 @@ __device__ __noinline__ uint32_t search_on(uint32_t hs, uint32_t cur, bool judge
   bool others = judge;  // the surge sets of other sizes are still to be closed
   for (uint32_t quiet = 0;;) {
     if (judge && surge_slabs_held(sid)) {
-      if (set_level(sid, 0)) red_add(&g_st.n_surge_changes, 1);
+      set_level(sid, 0);
       for (uint32_t k = 1; k < kMaxHeads; k++) retire_set(k * kNSizes + sid, true);
       closed = true;
     }
@@ -897,13 +915,11 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs, uint32_t crossed, boo
       settle(hs, next);
       return cur;
     }
-    const uint32_t level = judge ? head_level(wcur) : 0u;
-    uint32_t nlevel = level;
+    bool closed = false;
     if (next == kNone) next = find_slab(sid);
     if (next == kNone && !surge_set) {
-      bool closed = false, moved = false;
+      bool moved = false;
       next = search_on(hs, cur, judge, epoch, closed, moved);
-      if (closed) nlevel = 0;
       if (moved) {
         unlock(hlock);
         settle(hs, kNone);
@@ -917,8 +933,21 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs, uint32_t crossed, boo
       settle(hs, kNone);
       return none;
     }
-    const uint32_t wnew = head_word(next, nlevel);
-    const uint32_t was = head_slab(atom_exch(head, wnew));
+    // The level is the word's own: others may have opened or closed sets since
+    // it was read.  Every failed try is a change of another warp.
+    uint32_t w = wcur, wnew;
+    for (uint32_t i = 0;; i++) {
+      wnew = head_word(next, head_level(w));
+      const uint32_t now = atom_cas(head, w, wnew);
+      if (now == w) break;
+      w = now;
+      if (i == 1024) {
+        unlock(hlock);
+        settle(hs, next);
+        return head_slab(w);
+      }
+    }
+    const uint32_t was = head_slab(w);
     unlock(hlock);
     if (was != cur && was != kNone) {
       // another warp's change came in between: its head may not be busy yet
@@ -926,9 +955,9 @@ __device__ __noinline__ uint32_t replace_head(uint32_t hs, uint32_t crossed, boo
         retire(was);
         unlock(&g_st.sb_lock[was]);
       }
-      after_change(hs, kNone, wnew, judge && nlevel == level, group);
+      after_change(hs, kNone, wnew, judge && !closed, group);
     } else {
-      after_change(hs, was, wnew, judge && nlevel == level, group);
+      after_change(hs, was, wnew, judge && !closed, group);
     }
     return next;
   }

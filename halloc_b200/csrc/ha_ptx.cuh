@@ -106,6 +106,7 @@ __device__ __forceinline__ uint32_t atom_exch_acquire(uint32_t *p, uint32_t v) {
 __device__ __forceinline__ void fence_acq_rel() {
   asm volatile("fence.acq_rel.gpu;" ::: "memory");
 }
+__device__ __forceinline__ void fence_sc() { asm volatile("fence.sc.gpu;" ::: "memory"); }
 
 // Slab metadata accesses (bit arrays, size nibbles, slab counters) carry an
 // L2 evict-last cache policy, so that the metadata of the slabs in use stays

@@ -589,7 +589,7 @@ __global__ void ha_close_surges_k() {
   for (uint32_t sid = 0; sid < kNSizes; sid++) {
     uint32_t *hlock0 = &g_st.head_lock[sid * kTicketStride];
     if (lock(hlock0)) {
-      if (set_level(sid, 0)) red_add(&g_st.n_surge_changes, 1);
+      set_level(sid, 0);
       unlock(hlock0);
     }
     for (uint32_t k = 1; k < kMaxHeads; k++) retire_set(k * kNSizes + sid, true);

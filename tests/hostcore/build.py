@@ -96,3 +96,4 @@ class Core:
     nulls = property(lambda self: self.lib.hc_nulls())
     head_changes = property(lambda self: self.lib.hc_head_changes())
     surge_changes = property(lambda self: self.lib.hc_surge_changes())
+    level_moves = property(lambda self: self.lib.hc_level_moves())

@@ -34,6 +34,7 @@ uint64_t hc_time_ns();           // grows with every point
 uint32_t hc_lane();
 uint32_t hc_mask();              // the lanes of the calling lane's warp
 uint32_t hc_sm();
+void hc_wrote(const uint32_t *p, uint32_t from, uint32_t to);  // by a swap or an exchange
 // the values that the lanes of `mask` bring, once all have come
 const uint64_t *hc_meet(uint32_t mask, uint64_t value);
 
@@ -111,7 +112,7 @@ inline void st_release(uint32_t *p, uint32_t v) { hc_store(p, v); }
 HC_RMW(atom_add, uint32_t, o + v)
 HC_RMW(atom_or, uint32_t, o | v)
 HC_RMW(atom_and, uint32_t, o & v)
-HC_RMW(atom_exch, uint32_t, v)
+HC_RMW(exchanged, uint32_t, v)
 HC_RMW(atom_exch_acquire, uint32_t, v)
 HC_RMW(atom_add_meta, uint32_t, o + v)
 HC_RMW(atom_or_meta, uint32_t, o | v)
@@ -123,7 +124,16 @@ inline T hc_cas(T *p, T expect, T v) {
   if (o == expect) *p = v;
   return o;
 }
-inline uint32_t atom_cas(uint32_t *p, uint32_t expect, uint32_t v) { return hc_cas(p, expect, v); }
+inline uint32_t atom_cas(uint32_t *p, uint32_t expect, uint32_t v) {
+  const uint32_t o = hc_cas(p, expect, v);
+  if (o == expect) hc_wrote(p, o, v);
+  return o;
+}
+inline uint32_t atom_exch(uint32_t *p, uint32_t v) {
+  const uint32_t o = exchanged(p, v);
+  hc_wrote(p, o, v);
+  return o;
+}
 inline void red_add(uint32_t *p, uint32_t v) { atom_add(p, v); }
 inline void red_add_release(uint32_t *p, uint32_t v) { atom_add(p, v); }
 inline void red_or(uint32_t *p, uint32_t v) { atom_or(p, v); }
@@ -131,6 +141,7 @@ inline void red_and(uint32_t *p, uint32_t v) { atom_and(p, v); }
 inline void red_or_meta(uint32_t *p, uint32_t v) { atom_or(p, v); }
 inline void red_and_meta(uint32_t *p, uint32_t v) { atom_and(p, v); }
 inline void fence_acq_rel() {}
+inline void fence_sc() {}
 inline Desc ld_desc(const Desc *p) {
   Desc d;
   d.size_id = hc_load(&p->size_id);

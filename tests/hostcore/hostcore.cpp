@@ -55,6 +55,7 @@ Lane *g_cur = nullptr;
 jmp_buf g_main;
 uint64_t g_points = 0, g_rng = 1;
 uint32_t g_hold = 0;  // one point in g_hold holds its lane back (0: none)
+uint32_t g_level_moves = 0;  // changes of the level in a set-0 head word
 std::vector<uint32_t> g_meta;
 bool g_stuck = false;
 
@@ -115,6 +116,10 @@ void hc_pause(uint32_t ns) {
   g_cur->wake = g_points + ns / 20 + 1;
   to_main();
 }
+void hc_wrote(const uint32_t *p, uint32_t from, uint32_t to) {
+  if (p >= ha::g_st.head && p < ha::g_st.head + ha::kNSizes)
+    g_level_moves += ha::head_level(from) != ha::head_level(to);
+}
 uint64_t hc_time_ns() { return g_points * 20; }
 uint32_t hc_lane() { return g_cur->id; }
 uint32_t hc_mask() { return g_cur->warp->mask; }
@@ -156,6 +161,7 @@ void hc_init(uint32_t nsbs, uint32_t sb_sh, const uint32_t *cls, uint32_t nheads
              uint32_t spec_mask) {
   using namespace ha;
   memset(&g_st, 0, sizeof(g_st));
+  g_level_moves = 0;
   memset(&c_cfg, 0, sizeof(c_cfg));
   memcpy(g_cls, cls, sizeof(g_cls));
   for (uint32_t s = 0; s < kNSizes; s++) {
@@ -263,6 +269,7 @@ uint32_t hc_status() { return ha::g_st.status; }
 uint32_t hc_nulls() { return ha::g_st.n_null; }
 uint32_t hc_head_changes() { return ha::g_st.n_head_changes; }
 uint32_t hc_surge_changes() { return ha::g_st.n_surge_changes; }
+uint32_t hc_level_moves() { return g_level_moves; }
 // head slab, prefetched slab and level of head set k of size sid; the copy
 // of the level beside it
 void hc_head(uint32_t sid, uint32_t k, uint32_t out[4]) {

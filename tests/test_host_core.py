@@ -128,3 +128,22 @@ def test_a_slab_with_room_is_in_a_set(core, sizes, lanes, surge):
                         for _ in range(int(rng.integers(2, 12)))], seed)
         assert core.status == 0, seed
         assert_quiescent(core, res, seed)
+
+
+@pytest.mark.parametrize("sizes,lanes", [([2048], 4), ([256], 8), ([512, 768, 2048], 4)])
+def test_a_level_changes_only_where_it_is_judged(core, sizes, lanes):
+    """Warps storm sizes whose levels open and close: every change of the level
+    in a head word is one that was decided (and counted), and the copy of the
+    level beside it is right once the warps are done."""
+    moves = 0
+    for seed in range(250):
+        rng = np.random.default_rng(seed)
+        core.init(int(rng.integers(6, 40)))
+        core.run([churn(rng, int(rng.integers(20, 120)), lanes, sizes, rng.uniform(0.1, 0.5), 0.5)
+                  for _ in range(int(rng.integers(2, 12)))], seed)
+        assert core.status == 0 and core.level_moves == core.surge_changes, seed
+        for size in sizes:
+            h = core.head(SID[size])
+            assert h["level"] == h["level_copy"], (seed, size, h)
+        moves += core.level_moves
+    assert moves > 0
