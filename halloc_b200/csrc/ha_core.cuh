@@ -1410,18 +1410,24 @@ __device__ __forceinline__ void *malloc_small(uint32_t nbytes) {
   return p;
 }
 
-// Whether a count of n0 chunks lowered by n crosses a threshold of size sid
-// or empties the slab: only then is the slab filed anew.  sid is the size
-// that the descriptor showed at the start of the free; a slab whose size
-// changed meanwhile has the same chunk size, and thresholds that differ by
-// two chunks at most.  Saves file_after_free's own reads of the descriptor
-// (one more round trip) for nearly every free in a slab that is no head.
+// Whether a count of n0 chunks lowered by n may cross a threshold of the slab
+// or empties it: only then is the slab filed anew.  sid is the size that the
+// descriptor showed at the start of the free.  The slab's size may have changed
+// meanwhile, but not its chunk size, and thresholds of sizes with the same
+// chunks differ by less than kFilingSlack: they are fractions of the slab's
+// chunks rounded down to whole blocks, of eight chunks at most.  Within the
+// slack file_after_free compares with the slab's own.  Saves its reads of the
+// descriptor (one more round trip) for nearly every free in a slab that is no
+// head.
+constexpr uint32_t kFilingSlack = 8;
+__device__ __forceinline__ bool may_cross(uint32_t t, uint32_t n0, uint32_t n1) {
+  return n1 < t + kFilingSlack && n0 + kFilingSlack > t;
+}
 __device__ __forceinline__ bool crosses(uint32_t sid, uint32_t n0, uint32_t n) {
   if (sid >= kNSizes) return true;
   const uint4 b = __ldg(reinterpret_cast<const uint4 *>(&g_cls[sid]) + 1);
   const uint32_t n1 = n0 - n;  // b: sparse, hash_step, roomy, busy
-  return n1 == 0 || (n1 <= b.w && n0 > b.w) || (n1 <= b.z && n0 > b.z) ||
-         (n1 <= b.x && n0 > b.x);
+  return n1 == 0 || may_cross(b.w, n0, n1) || may_cross(b.z, n0, n1) || may_cross(b.x, n0, n1);
 }
 
 // Small-block free for every active lane of the calling warp; `off` is the

@@ -147,3 +147,20 @@ def test_a_level_changes_only_where_it_is_judged(core, sizes, lanes):
             assert h["level"] == h["level_copy"], (seed, size, h)
         moves += core.level_moves
     assert moves > 0
+
+
+@pytest.mark.parametrize("sb_sh", [16, 20, 21, 22, 23, 24])
+@pytest.mark.parametrize("fractions", [{}, {"busy": 0.91, "roomy": 0.5, "sparse": 0.0125}])
+def test_a_free_sees_the_thresholds_of_every_size_of_the_chunk(core, sb_sh, fractions):
+    """A slab's size may change, within its chunk size, between a free's reading
+    of the descriptor and the lowering of its count: whichever size it read,
+    the free has to notice that it takes the slab over a threshold."""
+    core.init(4, sb_sh=sb_sh, **fractions)
+    c = core.cls.astype(int)
+    for now in range(16):
+        for seen in (s for s in range(16) if c[s, 2] == c[now, 2]):
+            for t in c[now, [4, 6, 7]]:
+                for n in sorted({1, 2, 3, c[now, 3], 8 * c[now, 3], 32 * c[now, 3]}):
+                    for n0 in range(t + 1, min(t + n, c[now, 0]) + 1):
+                        if n0 >= n:
+                            assert core.lib.hc_crosses(int(seen), n0, int(n)), (now, seen, t, n0, n)
