@@ -599,11 +599,15 @@ __device__ __noinline__ bool close_other_surges(uint32_t own) {
 // Whether a size may open surge level `level`: more heads hold more partly
 // filled slabs, so only while a quarter of the pool is free.  The topmost
 // level, whose heads and prefetched slabs are 32, opens only in pools of at
-// least five times as many slabs, while half of them are free: 131 K threads
-// on sizes up to 3 KiB in a pool of 192 slabs went from 366 to 178 us with it
-// and a graph build from 348 to 329; in a pool of 96 slabs (256-B blocks from
-// 1 M threads) it ran the size short, 664 us against 573, and so did 32 sets
-// in the first.
+// least five times as many slabs, while half of them are free.  Without it and
+// with it, 131 K threads on sizes up to 3 KiB: 384 and 196 us a pass in a pool
+// of 160 slabs, 381 and 193 of 192, 381 and 190 of 256 -- but 398 and 4,008 of
+// 128, where it ran sizes short (144: 382 and, in two runs of six, 5,400); 256-B
+// blocks from 1 M threads: 530 and 456 of 160, 533 and 457 of 192, 549 and 471
+// of 384 -- but 529 and 583 of 96.  32 sets ran a pool of 192 short.
+// At 192 slabs the first has two modes: where a size that needs 16 sets less
+// opens them first, just under half of the pool is left, and a pass takes
+// 375 us (one run in six; with 7/16 free as the limit in none of six).
 __device__ __forceinline__ bool room_for_level(uint32_t level, uint32_t nfree,
                                                uint32_t committed) {
   if (level <= kWideLevel) return (uint64_t)kSurgeFreeOpen * nfree >= committed;
@@ -650,11 +654,10 @@ __device__ __forceinline__ uint32_t tickets_of(uint32_t sid) {
 // count.  Once the window is full (kProbeStormUp) that warp takes it
 // with an exchange and judges it: a level opens when the size gave out
 // fewer than kProbeStormTickets tickets per long probe since the window
-// began; either way a new window begins.  Only set 0's ticket counter is
-// read: with 2^level sets open it serves that fraction of the SMs, so its
-// count is scaled up by 2^level.  This function must stay a leaf (surge_open
-// is inlined): with a call to a non-inlined function here, a call that never
-// ran, that workload lost a third of its rate.
+// began, over all its counters; either way a new window begins.  This
+// function must stay a leaf (surge_open is inlined): with a call to a
+// non-inlined function here, a call that never ran, that workload lost a third
+// of its rate.
 __device__ __noinline__ void probe_storm(uint32_t sid, uint32_t k, uint32_t c) {
   uint32_t *line = &g_st.storm[sid * kTicketStride];
   red_add(line + 2, 8u * k);
@@ -675,8 +678,9 @@ __device__ __noinline__ void probe_storm(uint32_t sid, uint32_t k, uint32_t c) {
 
 // The surge level for size sid after a head of its set 0 was used up (set
 // `level` sets open so far), from how many warps queued for the size's heads
-// during the old head's life, how many tickets set 0 gave out meanwhile (about
-// the allocations its head served) and how long it lived.  A level opens when
+// during the old head's life, how many tickets set 0's counter gave out
+// meanwhile (about the allocations its head served; an SM with an old copy of
+// the level draws from another set's counter) and how long it lived.  A level opens when
 // the queue is a storm (kSurgeUp), or when it is long and the head served
 // only a few allocations per queued warp of its set (a head too small for the
 // grid: kSurgeTicketsUp each), or when a warp of several lanes (`group`) used up a
@@ -1302,7 +1306,9 @@ __device__ __forceinline__ void *malloc_small(uint32_t nbytes) {
   // along with set 0's, so that a storm costs no second round trip and its
   // tickets do not all pass through set 0's counter first (3,600 cycles for a
   // ticket with nine sizes in a warp).  A stale copy only draws the ticket
-  // from another counter; the head comes from the words as they are now.
+  // from another counter, whose first positions in a head may be those that the
+  // head's own counter gives out; the head comes from the words as they are now.
+  // (A load that drops the old copy from L1 whenever it was wrong changed nothing.)
   const uint32_t guess = ld_cached(&g_st.level[sid]);
   uint32_t w = ld_relaxed(&g_st.head[hs]);
   // the lanes of each size draw consecutive tickets, in lane order, with one

@@ -302,6 +302,11 @@ __device__ __forceinline__ unsigned long long read_sum(const void *p, uint32_t s
   return sum;
 }
 
+// Both phase rounds read a thread's slots four at a time, so that their DRAM
+// reads overlap instead of each waiting behind the slot before.  A free round
+// of 3.8 M blocks of 95 bytes on average: 383 us slot by slot, 253-268 so.
+constexpr uint32_t kSlotBatch = 4;
+
 // Phase accumulators: [0] slots filled after the round, [1] failed
 // allocations, [2] sum of words written, [3] sum of words read back,
 // [4] allocations, [5] frees.
@@ -309,11 +314,6 @@ __device__ __forceinline__ unsigned long long read_sum(const void *p, uint32_t s
 // One allocation round: every empty slot of every thread is filled with
 // probability thr / 2^32 by a block of a size drawn from size_set, whose
 // words are written with base, base+1, ...
-// Both rounds read a thread's slots four at a time, so that their DRAM reads
-// overlap instead of each waiting behind the slot before.  A free round of
-// 3.8 M blocks of 95 bytes on average: 383 us with that loop, 253-268 now.
-constexpr uint32_t kSlotBatch = 4;
-
 __global__ void __launch_bounds__(128, 8) ha_phase_alloc_k(uint32_t n, uint32_t nslots, uint32_t seed, uint32_t round,
                                  uint32_t thr, const uint32_t *size_set, uint32_t nsizes,
                                  void **slots, uint32_t *slot_sz, unsigned long long *acc) {

@@ -118,10 +118,13 @@ __device__ __forceinline__ uint32_t slab_bucket(const PointNode *p) {
 }
 
 // kWide: every warp of the block walks 32 lists, a quarter as deep, for grids of
-// many cells, whose lists are short and for which one walker per block means
-// four times the blocks: insert, walk and free of 1 M points in 64^3 cells took
-// 118 us with one walker and takes 87, of 1,000 points 21.9 and 20.2; in 32^3
-// cells the one walker is the quicker, 109 us.
+// many cells, which fill the GPU with walkers either way and for which one
+// walker per block means four times the blocks.  The line lies by the cells:
+// what counts is how many walkers there are, however long the lists.  The free
+// alone, one walker and all warps walking, in us: 1 M points in 24^3 cells 78
+// and 164, 32^3 53 and 87, 40^3 45 and 62, 48^3 41 and 50, 64^3 64-74 and 47,
+// 100^3 96 and 61; 4 M points in 40^3 211 and 211, 48^3 208 and 160, 64^3 (16
+// a cell) 201 and 152; 8 M points in 64^3 (32 a cell) 423 and 288.
 constexpr uint32_t kGridWide = 1u << 16;  // cells from which on every warp walks
 
 template <bool kWide>

@@ -108,9 +108,9 @@ constexpr uint32_t kSurgeQueueMin = 128;
 // third trigger, probing storms: lanes whose probe call needed
 // kLongProbeRounds or more look-ahead rounds in a slab under half its busy
 // threshold -- a head far from full whose first positions keep meeting taken
-// chunks.  kProbeStormUp of them while the size's set-0 counter gave out
-// fewer than kProbeStormTickets tickets each open a level at once (the head
-// may never fill, so no head change would come to decide it).
+// chunks.  kProbeStormUp of them while the size's counters gave out fewer
+// than kProbeStormTickets tickets each open a level at once (the head may
+// never fill, so no head change would come to decide it).
 #ifndef HA_PROBE_STORM
 #define HA_PROBE_STORM 1  // 0 builds without the third trigger
 #endif
@@ -197,8 +197,8 @@ struct State {
   // per size, one 128-B line: [0] warps that queued for the head lock since
   // the last change of its set-0 head, capped near kSurgeUp; [1] set 0's
   // ticket at that change; [2] long-probe lanes in the current probe-storm
-  // window; [3] set 0's ticket when that window began; [4] time of the last
-  // change of its set-0 head (units of 1,024 ns)
+  // window; [3] the tickets of all its counters when that window began; [4]
+  // time of the last change of its set-0 head (units of 1,024 ns)
   alignas(128) uint32_t storm[kNSizes * kTicketStride];
   alignas(128) uint32_t ctr[kMaxSlabs * kCtrStride];
   alignas(128) Desc desc[kMaxSlabs];

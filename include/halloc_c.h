@@ -374,8 +374,8 @@ int ha_grid_insert_c(uint32_t n, uint32_t ncells, const float *pts, void **grid,
    finaliser), into device arrays of ncells^3 entries. */
 int ha_grid_check_c(uint32_t ncells, void *const *grid, uint32_t *count, uint64_t *hsum,
                     void *stream);
-/* One thread per cell frees the cell's nodes (unless pre_nodes) and clears
-   the cell. */
+/* Clears every cell and, unless pre_nodes, frees its nodes: warps walk 32
+   cells' lists at a time, and the threads of a block free what they found. */
 int ha_grid_free_c(uint32_t ncells, void **grid, int pre_nodes, void *stream);
 
 /* add-strings (halloc samples/add-strings/add-strings.cu:71-205): string i
