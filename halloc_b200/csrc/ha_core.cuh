@@ -599,19 +599,25 @@ __device__ __noinline__ bool close_other_surges(uint32_t own) {
 // Whether a size may open surge level `level`: more heads hold more partly
 // filled slabs, so only while a quarter of the pool is free.  The topmost
 // level, whose heads and prefetched slabs are 32, opens only in pools of at
-// least five times as many slabs, while half of them are free.  Without it and
+// least five times as many slabs, while half of them are free, or three eighths
+// for sizes whose heads are small (kSmallHead).  Without it and
 // with it, 131 K threads on sizes up to 3 KiB: 384 and 196 us a pass in a pool
 // of 160 slabs, 381 and 193 of 192, 381 and 190 of 256 -- but 398 and 4,008 of
 // 128, where it ran sizes short (144: 382 and, in two runs of six, 5,400); 256-B
 // blocks from 1 M threads: 530 and 456 of 160, 533 and 457 of 192, 549 and 471
 // of 384 -- but 529 and 583 of 96.  32 sets ran a pool of 192 short.
-// At 192 slabs the first has two modes: where a size that needs 16 sets less
-// opens them first, just under half of the pool is left, and a pass takes
-// 375 us (one run in six; with 7/16 free as the limit in none of six).
-__device__ __forceinline__ bool room_for_level(uint32_t level, uint32_t nfree,
+// The small heads' own limit: with half for every size, a size that needs 16
+// sets less could open them first and leave the largest size just under half of
+// the pool; a pass of the first then took 375-390 us for good, in 12 of 24 runs
+// at 160 to 208 slabs, and in none with three eighths.  Three eighths for
+// every size opened levels in the phase workload that it does better without,
+// 2,020 us against 1,910.
+__device__ __forceinline__ bool room_for_level(uint32_t sid, uint32_t level, uint32_t nfree,
                                                uint32_t committed) {
   if (level <= kWideLevel) return (uint64_t)kSurgeFreeOpen * nfree >= committed;
-  return level <= kMaxLevel && committed >= (10u << level) && 2ull * nfree >= committed;
+  if (level > kMaxLevel || committed < (10u << level)) return false;
+  const bool small = __ldg(&g_cls[sid].nchunks) < kSmallHead * __ldg(&g_cls[sid].ncib);
+  return 8ull * nfree >= (small ? 3ull : 4ull) * committed;
 }
 
 // Opens one more surge level for size sid now, keeping set 0's head slab:
@@ -628,7 +634,7 @@ __device__ __forceinline__ void surge_open(uint32_t sid) {
   const uint32_t level = head_level(w);
   const uint32_t nfree = ld_relaxed(&g_st.n_free);
   const uint32_t committed = ld_relaxed(&g_st.committed);
-  if (head_slab(w) != kNone && room_for_level(level + 1, nfree, committed)) {
+  if (head_slab(w) != kNone && room_for_level(sid, level + 1, nfree, committed)) {
     if (atom_cas(head, w, head_word(head_slab(w), level + 1)) == w) {
       red_add(&g_st.n_surge_changes, 1);
       copy_level(sid);
@@ -704,7 +710,7 @@ __device__ __forceinline__ uint32_t judge_level(uint32_t sid, uint32_t level, bo
   const uint32_t nfree = ld_relaxed(&g_st.n_free);
   const uint32_t committed = ld_relaxed(&g_st.committed);
   const bool hot = group && life < kSurgeHotLife;
-  if ((storm >= kSurgeUp || crowded || hot) && room_for_level(level + 1, nfree, committed))
+  if ((storm >= kSurgeUp || crowded || hot) && room_for_level(sid, level + 1, nfree, committed))
     return level + 1;
   if (level > 0 && ((storm < kSurgeDown && calm && life >= kSurgeCalmLife) ||
                     (uint64_t)kSurgeFreeClose * nfree < committed))

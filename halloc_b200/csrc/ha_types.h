@@ -105,6 +105,9 @@ constexpr uint32_t kSurgeQueueMin = 128;
 #ifndef HA_SURGE_FREE_CLOSE
 #define HA_SURGE_FREE_CLOSE 8
 #endif
+// blocks of a head under which a size counts as one of small heads (1.5 KiB and
+// more with 4 MiB slabs)
+constexpr uint32_t kSmallHead = 4096;
 // third trigger, probing storms: lanes whose probe call needed
 // kLongProbeRounds or more look-ahead rounds in a slab under half its busy
 // threshold -- a head far from full whose first positions keep meeting taken

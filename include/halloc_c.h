@@ -173,7 +173,8 @@ int ha_set_heads_c(uint32_t nheads);
    two or more look-ahead rounds within 16 tickets each), the size gets 2,
    then 4, then 8 head slabs, each serving the SMs whose id modulo the set
    count names it -- while a quarter of the pool's slabs is free -- and 16 in a
-   pool of at least 160 slabs, half of them free.
+   pool of at least 160 slabs, half of them free (three eighths for sizes
+   whose heads hold fewer than 4,096 blocks).
    The sets close again one level per calm head change, after a head that
    lived a millisecond (or while under an eighth of the pool is free), and
    all of them at once when a size runs short of slabs, so a NULL still means
