@@ -270,6 +270,10 @@ uint32_t hc_nulls() { return ha::g_st.n_null; }
 uint32_t hc_head_changes() { return ha::g_st.n_head_changes; }
 uint32_t hc_surge_changes() { return ha::g_st.n_surge_changes; }
 uint32_t hc_level_moves() { return g_level_moves; }
+// whether size sid may open surge level `level`
+uint32_t hc_room(uint32_t sid, uint32_t level, uint32_t nfree, uint32_t committed) {
+  return ha::room_for_level(sid, level, nfree, committed);
+}
 // whether a free looks at the sets of a slab whose descriptor showed size sid
 uint32_t hc_crosses(uint32_t sid, uint32_t n0, uint32_t n) { return ha::crosses(sid, n0, n); }
 // head slab, prefetched slab and level of head set k of size sid; the copy

@@ -164,3 +164,22 @@ def test_a_free_sees_the_thresholds_of_every_size_of_the_chunk(core, sb_sh, frac
                     for n0 in range(t + 1, min(t + n, c[now, 0]) + 1):
                         if n0 >= n:
                             assert core.lib.hc_crosses(int(seen), n0, int(n)), (now, seen, t, n0, n)
+
+
+@pytest.mark.parametrize("sb_sh", [20, 22, 24])
+def test_the_topmost_level_opens_by_pool_and_head_size(core, sb_sh):
+    """Levels 1 to 3 need a quarter of the pool free; level 4 a pool of 160 slabs
+    with half of them free, or three eighths where a head holds fewer than 4,096
+    blocks, which depends on the size and on the slabs."""
+    core.init(4, sb_sh=sb_sh)
+    room = core.lib.hc_room
+    for sid in range(16):
+        blocks = int(core.cls[sid, 0]) // int(core.cls[sid, 3])
+        for committed in (159, 160, 192, 1000):
+            for level in (1, 3, 4, 5):
+                for nfree in range(committed + 1):
+                    want = 4 * nfree >= committed
+                    if level >= 4:
+                        eighths = 3 if blocks < 4096 else 4
+                        want = level == 4 and committed >= 160 and 8 * nfree >= eighths * committed
+                    assert bool(room(sid, level, nfree, committed)) == want, (sid, level, nfree)
